@@ -24,6 +24,7 @@
 #include "kernels.cuh"
 #include "anderson.cuh"
 #include "control.cuh"
+#include "linked.cuh"
 #include "shapes.cuh"
 
 namespace pdlpx {
@@ -334,6 +335,15 @@ __global__ void __launch_bounds__(kBlock, sellMinBlocks<float, true>())
     primalSellFrom<U, float, ST, false, true>(p, idx, val, begin + r, hdr[r / kSlice], koff);
 }
 
+// ---- linked restart cycle (linked.cuh) ------------------------------------------
+// 16 warps at 128 registers; with CSR rows, whose eight sums per lane would
+// spill there, 8 warps.
+constexpr int linkThreads(bool csr) { return csr ? 256 : 512; }
+template <int LP, int LD, bool CSR, class T>
+__global__ void __launch_bounds__(linkThreads(CSR), 1) linkedSteps(LinkArgs<T> a) {
+    linkedCycle<LP, LD, CSR, T>(a);
+}
+
 // ---- power iteration over the sliced-ELL sides --------------------------------
 // The short rows of A (y = A x) and of A^T (x_n = A^T y, with the block
 // partials of x . x_n and x_n . x_n) in the step kernels' layout: one thread
@@ -405,6 +415,14 @@ int32_t pickGroup(int64_t nnz, int32_t rows) {
 // ---------------------------------------------------------------------------
 // Device image
 // ---------------------------------------------------------------------------
+// What the host reads after a cycle: the solver state, the linked cycle's step
+// times and whether one of its waits ran out.
+struct StateBlock {
+    DevState st;
+    LinkTime lt;
+    int link_err;
+};
+
 struct DeviceLp {
     int device = 0;
     int sms = 148;
@@ -485,16 +503,25 @@ struct DeviceLp {
     DevState* h_st = nullptr;    // pinned mirror
     PowerState* h_ps = nullptr;  // pinned mirror
 
-    cudaGraphExec_t cycle[2] = {nullptr, nullptr};
-    int cycle_N[2] = {0, 0};
+    // linked restart cycle (linked.cuh): whether it runs the steps, lanes per
+    // sliced-ELL column
+    bool linked = false;
+    int link_lanes = 4;
+    int link_warps = 0;  // of its grid per SM
+    void *link_x = nullptr, *link_y = nullptr;  // cells (null: the launches run)
+
+    // [FP32 / FP64][step launches / linked]
+    cudaGraphExec_t cycle[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
+    int cycle_N[2][2] = {{0, 0}, {0, 0}};
     cudaGraphExec_t power = nullptr;
-    int launches_cycle[2] = {0, 0};
+    int launches_cycle[2][2] = {{0, 0}, {0, 0}};
     int launches_power = 0;
     static constexpr int kPowerChunk = 8;
 
     ~DeviceLp() {
-        for (auto& g : cycle)
-            if (g) cudaGraphExecDestroy(g);
+        for (auto& row : cycle)
+            for (auto& g : row)
+                if (g) cudaGraphExecDestroy(g);
         for (auto& row : kev)
             for (auto& e : row)
                 if (e) cudaEventDestroy(e);
@@ -805,6 +832,128 @@ int launchDual(const DeviceLp& d, const IterArgs<T>& ia, int k, cudaStream_t s) 
     }
     return n;
 }
+// A matrix side as the linked cycle walks it.
+template <class T>
+LinkSide<T> linkSide(const DeviceLp& d, const IterArgs<T>& ia, bool primal) {
+    LinkSide<T> a{};
+    const int shape = primal ? d.shapeP : d.shapeD, lshape = primal ? d.shapeLP : d.shapeLD;
+    a.hdr = primal ? d.sp_hdr : d.sd_hdr;
+    a.idx = primal ? d.sp_idx : d.sd_idx;
+    a.val = sellVals<T>(d, primal);
+    a.ptr = primal ? ia.at_ptr : ia.a_ptr;
+    a.cidx = primal ? ia.at_idx : ia.a_idx;
+    a.cval = primal ? ia.at_val : ia.a_val;
+    a.rows = primal ? d.n : d.m;
+    a.nl = primal ? d.nlP : d.nlD;
+    a.lanes = isSell(shape) ? 0 : kShapes[shape].G;
+    a.unroll = isSell(shape) ? 0 : kShapes[shape].U;
+    a.llanes = kShapes[lshape].G;
+    a.lunroll = kShapes[lshape].U;
+    return a;
+}
+
+// Whether the linked cycle runs the steps of an LP, and with how many lanes per
+// sliced-ELL column (link_lanes).  Measured on B200 (us per iteration with check,
+// restart and power iteration, launches -> linked; random LPs have 8 entries per
+// column and 20 per row):
+//  * sliced ELL on both sides: 400 x 1,000 7.9 -> 3.3, 2,000 x 5,000 9.0 -> 4.3,
+//    20,000 x 50,000 14.2 -> 12.3, 30,000 x 75,000 (600k entries) 17.5 -> 15.5,
+//    40,000 x 100,000 23.0 -> 22.5: up to 600k entries.  4 lanes per column (8 per
+//    row) to 240k entries (12,000 x 30,000 9.6 against 10.0 with 2 and 4), above
+//    that 2 (20,000 x 50,000 12.3 against 14.1: more warps than an SM holds).
+//    Columns of up to 3 entries take one lane (transportation 30 x 40: 2.6
+//    against 2.8), long ones 8.
+//  * long rows beside sliced ELL: power law 2,000 x 8,000 20.4 -> 10.8, 8,000 x
+//    32,000 (321k entries) 37 -> 30, 25,000 x 100,000 (1.0M) 37 -> 50: to 400k.
+//  * a CSR side: transportation 97 x 131 (25k entries) 5.7 -> 3.9, 150 x 150 5.7 ->
+//    5.4, 200 x 200 (80k) 5.9 -> 5.8, 300 x 300 7.2 -> 7.8: to 60k.
+// Options that pin a launch shape keep the launches.
+bool linkCsr(const DeviceLp& d) { return !isSell(d.shapeP) || !isSell(d.shapeD) || d.nlP > 0 || d.nlD > 0; }
+bool linkable(const DeviceLp& d, const pdlpx_options& o) {
+    if (d.lt_C > 0 || o.hot_cache > 0) return false;
+    if (o.shape_primal > 0 || o.shape_dual > 0 || o.spmv_group_a > 0 || o.spmv_group_at > 0) return false;
+    const bool csr = !isSell(d.shapeP) || !isSell(d.shapeD);
+    return d.nnz <= (csr ? 60000 : (d.nlP > 0 || d.nlD > 0) ? 400000 : 600000);
+}
+void planLinked(DeviceLp& d) {
+    // rowDotU with two sums per lane (the autotuner may pick it) has no linked form
+    auto supported = [](int shape) { return isSell(shape) || kShapes[shape].U >= kLinkU; };
+    d.linked = d.link_x != nullptr && supported(d.shapeP) && supported(d.shapeD);
+    if (!d.linked) return;
+    const double mean = static_cast<double>(d.nnz - d.zlP) / std::max(1, d.n - d.nlP);
+    d.link_lanes = mean <= 3.0 ? 1 : mean > 14.0 ? 8 : d.nnz <= 240000 ? 4 : 2;
+    const bool csr = linkCsr(d);
+    const int lanes_p = csr && d.link_lanes != 1 ? 4 : d.link_lanes;
+    const int lanes_d = csr || d.link_lanes == 1 || d.link_lanes == 4 ? 8 : 4;
+    // one warp per unit over all SMs first (a unit's gathers queue in its SM's
+    // L1), and no wider blocks than that takes: small LPs leave room for the
+    // grids of other solvers
+    const int units = linkUnits(d.n, d.nlP, isSell(d.shapeP) ? 0 : kShapes[d.shapeP].G, lanes_p) +
+                      linkUnits(d.m, d.nlD, isSell(d.shapeD) ? 0 : kShapes[d.shapeD].G, lanes_d);
+    d.link_warps = std::min(linkThreads(csr) / 32, (units + d.sms - 1) / d.sms);
+}
+
+// Warps per SM of the linked grids that the solves running on a device would
+// launch, by device.  Above kLinkShare of them a cycle runs by launches, which
+// share the SMs better than waiting grids do (16 solver threads on one B200, us
+// per LP-iteration of all: 2,000 x 5,000 launches 0.80, linked 2.05; with 4
+// threads 2.44 and 2.15).  Both give the same bits, so the choice is made anew
+// for every cycle.
+constexpr int kLinkShare = 32;
+std::atomic<int> g_link_warps[64];
+struct LinkShare {
+    std::atomic<int>* total = nullptr;
+    int warps = 0;
+    LinkShare(int device, int w) {
+        if (w <= 0 || device < 0 || device >= 64) return;
+        total = &g_link_warps[device];
+        warps = w;
+        total->fetch_add(warps, std::memory_order_relaxed);
+    }
+    ~LinkShare() {
+        if (total) total->fetch_sub(warps, std::memory_order_relaxed);
+    }
+    LinkShare(const LinkShare&) = delete;
+    LinkShare& operator=(const LinkShare&) = delete;
+    bool fits() const { return total != nullptr && total->load(std::memory_order_relaxed) <= std::max(kLinkShare, warps); }
+};
+
+template <int LP, int LD, bool CSR, class T>
+cudaError_t launchLinkedAs(const DeviceLp& d, LinkArgs<T>& a, cudaStream_t s) {
+    a.P.units = linkUnits(a.P.rows, a.P.nl, a.P.lanes, LP);
+    a.D.units = linkUnits(a.D.rows, a.D.nl, a.D.lanes, LD);
+    const int units = a.P.units + a.D.units;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(std::min(d.sms, (units + d.link_warps - 1) / d.link_warps)));
+    cfg.blockDim = dim3(static_cast<unsigned>(32 * d.link_warps));
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, linkedSteps<LP, LD, CSR, T>, a);
+}
+template <class T>
+cudaError_t launchLinked(const DeviceLp& d, const IterArgs<T>& ia, cudaStream_t s) {
+    LinkArgs<T> a{};
+    a.it = ia;
+    a.P = linkSide<T>(d, ia, true);
+    a.D = linkSide<T>(d, ia, false);
+    a.x = static_cast<LinkCell<T>*>(d.link_x);
+    a.y = static_cast<LinkCell<T>*>(d.link_y);
+    a.err = &reinterpret_cast<StateBlock*>(d.st)->link_err;
+    a.time = &reinterpret_cast<StateBlock*>(d.st)->lt;
+    if (linkCsr(d))
+        return d.link_lanes == 1 ? launchLinkedAs<1, 8, true, T>(d, a, s) : launchLinkedAs<4, 8, true, T>(d, a, s);
+    switch (d.link_lanes) {
+        case 1: return launchLinkedAs<1, 8, false, T>(d, a, s);
+        case 2: return launchLinkedAs<2, 4, false, T>(d, a, s);
+        case 4: return launchLinkedAs<4, 8, false, T>(d, a, s);
+        default: return launchLinkedAs<8, 4, false, T>(d, a, s);
+    }
+}
+
 // FP64 check pass: short rows write partials [0, nb_*_s), long rows the rest.
 template <class T>
 int launchChecks(const DeviceLp& d, const CheckArgs<T>& ca, cudaStream_t s) {
@@ -824,7 +973,7 @@ int launchChecks(const DeviceLp& d, const CheckArgs<T>& ca, cudaStream_t s) {
 
 // One restart cycle: N fused iterations, check, controller, restart copy.
 template <class T>
-int launchCycle(DeviceLp& d, const pdlpx_options& o) {
+int launchCycle(DeviceLp& d, const pdlpx_options& o, bool linked) {
     const IterArgs<T> ia = iterArgs<T>(d, o);
     const CheckArgs<T> ca = d.check<T>(ia.xh, ia.xi, ia.yh, ia.yi);
     cudaStream_t s = d.stream;
@@ -834,7 +983,11 @@ int launchCycle(DeviceLp& d, const pdlpx_options& o) {
     // becomes an event-record node of the graph (a plain record would only
     // mark a dependency), so every replay records it on the device.
     auto mark = [&](cudaEvent_t e) { cudaEventRecordWithFlags(e, s, cudaEventRecordExternal); };
-    for (int k = 1; k <= o.termination_eval_frequency; ++k) {
+    if (linked) {
+        launchLinked<T>(d, ia, s);
+        ++launches;
+    }
+    for (int k = 1; !linked && k <= o.termination_eval_frequency; ++k) {
         const bool timed = k == d.kev_iter && d.kev[p][0] != nullptr;
         if (timed) mark(d.kev[p][0]);
         launches += launchPrimal<T>(d, ia, k, s);
@@ -1350,6 +1503,9 @@ static int32_t buildDevice(std::unique_ptr<DeviceLp>& dp, const ScaledLp& sc_in,
     const size_t o_prev_ax = adaptive ? take(8 * m) : 0, o_prev_xh = adaptive ? take(8 * n) : 0;
     const size_t o_pi_x = take(8 * n), o_pi_y = take(8 * m), o_pi_xn = take(8 * n),
                  o_pi_part = take(8 * 2 * d.nb_pi);
+    // cells of the linked cycle
+    const bool link = linkable(d, o);
+    const size_t o_lx = link ? take(sizeof(LinkCell<double>) * n) : 0, o_ly = link ? take(sizeof(LinkCell<double>) * m) : 0;
     const size_t o_prow = take(8 * kRowSlots * d.nb_rows), o_pcol = take(8 * kColSlots * d.nb_cols);
     // sliced-ELL sides: slice headers, indices, FP64 values, FP32 values (mixed)
     const size_t eP = hsP.idx.size(), eD = hsD.idx.size();
@@ -1379,11 +1535,11 @@ static int32_t buildDevice(std::unique_ptr<DeviceLp>& dp, const ScaledLp& sc_in,
         o_aa[6] = take(4 * w);
         o_aa[7] = take(sizeof(AaState));
     }
-    const size_t o_st = take(sizeof(DevState)), o_dc = take(sizeof(DevConst)), o_ps = take(sizeof(PowerState));
+    const size_t o_st = take(sizeof(StateBlock)), o_dc = take(sizeof(DevConst)), o_ps = take(sizeof(PowerState));
     d.arena_bytes = off;
     const auto tb1 = std::chrono::steady_clock::now();
     PDLPX_CK(cudaMalloc(reinterpret_cast<void**>(&d.arena), d.arena_bytes));
-    PDLPX_CK(cudaMallocHost(reinterpret_cast<void**>(&d.h_st), sizeof(DevState)));
+    PDLPX_CK(cudaMallocHost(reinterpret_cast<void**>(&d.h_st), sizeof(StateBlock)));
     PDLPX_CK(cudaMallocHost(reinterpret_cast<void**>(&d.h_ps), sizeof(PowerState)));
     char* b = d.arena;
     d.a_ptr = reinterpret_cast<int*>(b + o_a_ptr);
@@ -1465,6 +1621,10 @@ static int32_t buildDevice(std::unique_ptr<DeviceLp>& dp, const ScaledLp& sc_in,
         d.aa_st = reinterpret_cast<AaState*>(b + o_aa[7]);
     }
     d.st = reinterpret_cast<DevState*>(b + o_st);
+    if (link) {
+        d.link_x = b + o_lx;
+        d.link_y = b + o_ly;
+    }
     d.dc = reinterpret_cast<DevConst*>(b + o_dc);
     d.ps = reinterpret_cast<PowerState*>(b + o_ps);
 
@@ -2097,21 +2257,30 @@ int32_t Engine::solveDevice(pdlpx_result* out) {
         PDLPX_CK(cudaMemsetAsync(d.prev_xh, 0, 8 * static_cast<size_t>(n), s));
     }
 
+    planLinked(d);
+    PDLPX_CK(cudaMemsetAsync(&reinterpret_cast<StateBlock*>(d.st)->link_err, 0, sizeof(int), s));
+    if (d.linked) {
+        PDLPX_CK(cudaMemsetAsync(d.link_x, 0, sizeof(LinkCell<double>) * static_cast<size_t>(n), s));
+        PDLPX_CK(cudaMemsetAsync(d.link_y, 0, sizeof(LinkCell<double>) * static_cast<size_t>(m), s));
+    }
     // ---- capture the restart-cycle graphs lazily
-    auto ensureCycle = [&](int prec) -> int32_t {
-        if (d.cycle[prec] && d.cycle_N[prec] == N) return PDLPX_OK;
-        if (d.cycle[prec]) {
-            cudaGraphExecDestroy(d.cycle[prec]);
-            d.cycle[prec] = nullptr;
+    const LinkShare link_share(d.device, d.linked ? d.link_warps : 0);
+    auto ensureCycle = [&](int prec, int link) -> int32_t {
+        cudaGraphExec_t& exec = d.cycle[prec][link];
+        if (exec && d.cycle_N[prec][link] == N) return PDLPX_OK;
+        if (exec) {
+            cudaGraphExecDestroy(exec);
+            exec = nullptr;
         }
         cudaGraph_t g = nullptr;
         PDLPX_CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-        d.launches_cycle[prec] = prec == 0 ? launchCycle<float>(d, opt_) : launchCycle<double>(d, opt_);
+        d.launches_cycle[prec][link] =
+            prec == 0 ? launchCycle<float>(d, opt_, link != 0) : launchCycle<double>(d, opt_, link != 0);
         PDLPX_CK(cudaStreamEndCapture(s, &g));
-        const cudaError_t ie = cudaGraphInstantiate(&d.cycle[prec], g, 0);
+        const cudaError_t ie = cudaGraphInstantiate(&exec, g, 0);
         cudaGraphDestroy(g);
         PDLPX_CK(ie);
-        d.cycle_N[prec] = N;
+        d.cycle_N[prec][link] = N;
         return PDLPX_OK;
     };
 
@@ -2130,14 +2299,28 @@ int32_t Engine::solveDevice(pdlpx_result* out) {
             stopped = true;
             break;
         }
-        const int32_t rc = ensureCycle(prec);
+        const int link = d.linked && link_share.fits() ? 1 : 0;
+        const int32_t rc = ensureCycle(prec, link);
         if (rc != PDLPX_OK) return rc;
-        PDLPX_CK(cudaGraphLaunch(d.cycle[prec], s));
-        launches += d.launches_cycle[prec];
-        PDLPX_CK(cudaMemcpyAsync(d.h_st, d.st, sizeof(DevState), cudaMemcpyDeviceToHost, s));
+        PDLPX_CK(cudaGraphLaunch(d.cycle[prec][link], s));
+        launches += d.launches_cycle[prec][link];
+        PDLPX_CK(cudaMemcpyAsync(d.h_st, d.st, sizeof(StateBlock), cudaMemcpyDeviceToHost, s));
         PDLPX_CK(cudaStreamSynchronize(s));
         const DevState& h = *d.h_st;
-        if (h.total - prev_total >= d.kev_iter) {
+        if (reinterpret_cast<const StateBlock*>(d.h_st)->link_err != 0) {
+            err = "linked cycle: a wait ran out of polls";
+            return PDLPX_E_TIMEOUT;
+        }
+        if (link) {
+            const LinkTime& q = reinterpret_cast<const StateBlock*>(d.h_st)->lt;
+            const double clk = static_cast<double>(q.primal_clk + q.dual_clk);
+            if (h.total > prev_total && q.iters > 0 && clk > 0.0) {
+                const double ms = 1e-6 * static_cast<double>(q.ns) / q.iters;
+                step_ms_[prec][0] += ms * static_cast<double>(q.primal_clk) / clk;
+                step_ms_[prec][1] += ms * static_cast<double>(q.dual_clk) / clk;
+                ++step_samples_[prec];
+            }
+        } else if (h.total - prev_total >= d.kev_iter) {
             // the timed iteration ran in full: read the step kernels' events of this cycle
             float a = 0.0f, b = 0.0f;
             if (cudaEventElapsedTime(&a, d.kev[prec][0], d.kev[prec][1]) == cudaSuccess &&

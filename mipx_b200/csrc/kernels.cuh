@@ -393,33 +393,42 @@ constexpr StepShape kShapes[] = {
 };
 constexpr int kNumShapes = sizeof(kShapes) / sizeof(kShapes[0]);
 
-// Halpern primal step of column j given s = (A^T y_cur)_j: projected gradient
-// step, reflection, averaging with the anchor (pdlp_kernels.cu:46-88).  FP64
-// arithmetic with the reference's association (tau = step * tau_base / omega).
+// Values of the Halpern primal step of a column given s = (A^T y_cur)_j:
+// projected gradient step (xh), reflection (xr), averaging with the anchor
+// (returned: the new current x) (pdlp_kernels.cu:46-88).  FP64 arithmetic with
+// the reference's association (tau = step * tau_base / omega).
 template <class T>
-__device__ __forceinline__ void primalUpdate(const IterArgs<T>& p, int j, const ColPack<T>& q, double xcd, double xid,
-                                             double s, double step, double pw, double lam, bool last) {
-    const double tau = step * static_cast<double>(q.tau) / pw;
-    double xh = xcd - tau * (static_cast<double>(q.c) + s);
+__device__ __forceinline__ double primalValues(const ColPack<T>& q, double xcd, double xid, double s, double tau,
+                                               double lam, double& xh, double& xr) {
+    xh = xcd - tau * (static_cast<double>(q.c) + s);
     const double lb = q.lb, ub = q.ub;
     if (xh < lb) xh = lb;
     if (xh > ub) xh = ub;
-    const double xr = 2.0 * xh - xcd;
+    xr = 2.0 * xh - xcd;
+    return lam * xr + (1.0 - lam) * xid;
+}
+
+template <class T>
+__device__ __forceinline__ void primalUpdate(const IterArgs<T>& p, int j, const ColPack<T>& q, double xcd, double xid,
+                                             double s, double step, double pw, double lam, bool last) {
+    double xh, xr;
+    const double xn =
+        primalValues<T>(q, xcd, xid, s, step * static_cast<double>(q.tau) / pw, lam, xh, xr);
     p.xr[j] = static_cast<T>(xr);
-    p.xc[j] = lam * xr + (1.0 - lam) * xid;
+    p.xc[j] = xn;
     if (last) p.xh[j] = static_cast<T>(xh);
 }
 
-// Dual proximal step of row i given s = (A x_refl)_i (pdlp_kernels.cu:94-157):
-// the projection of y + sigma (A x_refl) by row type, reflection, averaging.
+// Values of the dual proximal step of a row given s = (A x_refl)_i
+// (pdlp_kernels.cu:94-157): the projection of y + sigma (A x_refl) by row type
+// (py), reflection, averaging (returned: the new current y).
 template <class T>
-__device__ __forceinline__ void dualUpdate(const IterArgs<T>& p, int i, const RowPack<T>& q, double ycd, double yid,
-                                           double s, double step, double pw, double lam, bool last) {
+__device__ __forceinline__ double dualValues(const RowPack<T>& q, double ycd, double yid, double s, double step,
+                                             double pw, double lam, double& py) {
     const double sig = step * static_cast<double>(q.sigma) * pw;
     const double v = ycd + sig * s;
     const double rl = q.rl, ru = q.ru;
     const int type = static_cast<int>(q.type);
-    double py;
     if (type == 0) {
         py = v - sig * rl;
     } else if (type == 1) {
@@ -437,7 +446,14 @@ __device__ __forceinline__ void dualUpdate(const IterArgs<T>& p, int i, const Ro
             py = 0.0;
     }
     const double yr = 2.0 * py - ycd;
-    const double yn = lam * yr + (1.0 - lam) * yid;
+    return lam * yr + (1.0 - lam) * yid;
+}
+
+template <class T>
+__device__ __forceinline__ void dualUpdate(const IterArgs<T>& p, int i, const RowPack<T>& q, double ycd, double yid,
+                                           double s, double step, double pw, double lam, bool last) {
+    double py;
+    const double yn = dualValues<T>(q, ycd, yid, s, step, pw, lam, py);
     p.yc[i] = yn;
     if constexpr (sizeof(T) == 4) {
         if (p.yg != nullptr) p.yg[i] = static_cast<float>(yn);

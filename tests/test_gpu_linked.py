@@ -1,0 +1,139 @@
+"""The linked restart cycle (csrc/linked.cuh) against the step launches.
+
+Both sum every row in the same order and update it by the same expressions, so
+iterations, objective, x and y are the same bits.  The launches run where a
+launch shape is pinned; a pinned sliced-ELL variant (17: 4 entries per round)
+or the row-length table's own CSR shape (10: 32 lanes) changes no sum.
+"""
+import threading
+
+import numpy as np
+import pytest
+
+from mipx_b200 import generators as G
+from mipx_b200.pdlp import LpProblem, PdlpOptions, PdlpSolver, Precision, SparseMatrix
+
+pytestmark = pytest.mark.gpu
+
+LOOSE = dict(verbose=False, primal_tol=1e-4, dual_tol=1e-4, optimality_tol=1e-4, enable_polishing=False)
+
+# of the last check, so they tell the iterates apart where a capped solve returns no x
+FIELDS = ("status", "iterations", "restarts", "objective", "primal_objective", "dual_objective", "rel_primal_resid",
+          "rel_dual_resid", "primal_weight", "step_size", "fp64_iterations")
+
+
+def _solve(lp, **kw):
+    s = PdlpSolver()
+    s.setOptions(PdlpOptions(**{**LOOSE, **kw}))
+    s.load(lp)
+    r = s.solve()
+    return r, s
+
+
+def _same(lp, pins, **kw):
+    a, sa = _solve(lp, **kw)
+    b, sb = _solve(lp, **pins, **kw)
+    assert a.kernel_launches < b.kernel_launches, "the linked cycle did not run"
+    for f in FIELDS:
+        assert getattr(a, f) == getattr(b, f), f
+    np.testing.assert_array_equal(sa.getPrimalValues(), sb.getPrimalValues())
+    np.testing.assert_array_equal(sa.getDualValues(), sb.getDualValues())
+
+
+SELL = dict(shape_primal=17, shape_dual=17)
+
+
+def _holes(m, n, seed):
+    """Rows and columns without entries among rows of 0-40 entries."""
+    rng = np.random.default_rng(seed)
+    lens = np.where(rng.random(m) < 0.3, 0, rng.integers(1, min(n, 40) + 1, m))
+    ci = [np.sort(rng.choice(max(1, n - 3), size=min(k, max(1, n - 3)), replace=False)) for k in lens]
+    rp = np.concatenate([[0], np.cumsum([c.size for c in ci])]).astype(np.int32)
+    ci = np.concatenate(ci + [np.zeros(0, int)]).astype(np.int32)
+    v = rng.standard_normal(ci.size)
+    x0 = rng.uniform(0, 10, n)
+    ax = np.zeros(m)
+    np.add.at(ax, np.repeat(np.arange(m), np.diff(rp)), v * x0[ci])
+    return LpProblem(num_cols=n, num_rows=m, obj=rng.standard_normal(n), col_lower=np.zeros(n),
+                     col_upper=np.full(n, 10.0), row_lower=np.where(np.arange(m) % 3 == 0, ax, -np.inf),
+                     row_upper=ax + np.where(np.arange(m) % 3 == 0, 0.0, 1.0),
+                     matrix=SparseMatrix(m, n, values=v, col_indices=ci, row_starts=rp))
+
+
+# sizes around a warp's rows with 2, 4 and 8 lanes per row and around a slice,
+# columns longer than rows, one-entry LPs, and more units than the grid has warps
+@pytest.mark.parametrize("m,n,lo,hi", [(1, 1, 1, 1), (3, 7, 1, 2), (8, 9, 1, 8), (31, 33, 2, 9), (33, 64, 4, 12),
+                                       (257, 640, 4, 12), (900, 300, 18, 40), (1013, 2531, 4, 12), (5000, 12500, 1, 3),
+                                       (14000, 35000, 4, 12)])
+@pytest.mark.parametrize("precision", [Precision.FP64, Precision.Mixed])
+def test_sliced_ell(m, n, lo, hi, precision):
+    lp, _ = G.random_lp(m, n, lo, hi, 40 + m)
+    _same(lp, SELL, precision=precision, fp64_switch=precision == Precision.FP64, max_iter=1500)
+
+
+@pytest.mark.parametrize("m,n", [(5, 40), (64, 50), (700, 900)])
+def test_empty_rows_and_columns(m, n):
+    _same(_holes(m, n, m), SELL, max_iter=1000)
+
+
+@pytest.mark.parametrize("s,d", [(70, 80), (97, 131), (130, 180)])
+@pytest.mark.parametrize("fp32", [False, True])
+def test_csr_rows(s, d, fp32):
+    lp, _ = G.transport_lp(s, d, 3)
+    pins = dict(shape_primal=17, shape_dual=10 if lp.matrix.numNonzeros() / (s + d) <= 128 else 12)
+    _same(lp, pins, fp64_switch=not fp32, max_iter=1000)
+
+
+@pytest.mark.parametrize("m,kmax", [(1500, 100), (1500, 300), (3000, 700), (3000, 2000)])
+def test_long_columns(m, kmax):
+    lp, _ = G.powerlaw_lp(m, 4 * m, kmax=kmax, seed=m + kmax)
+    _same(lp, SELL, max_iter=1000)
+    _same(lp, SELL, max_iter=600, fp64_switch=False)
+
+
+# cycles cut short by the iteration limit, one iteration per cycle, restarts that
+# write y between cycles, the FP32 -> FP64 hand-over and the polish phase
+@pytest.mark.parametrize("kw", [dict(max_iter=777), dict(termination_eval_frequency=1, max_iter=60),
+                                dict(termination_eval_frequency=7, max_iter=400), dict(adaptive_step=True),
+                                dict(anderson_acceleration=True), dict(precision=Precision.FP64),
+                                dict(primal_tol=1e-5, dual_tol=1e-5, optimality_tol=1e-5, enable_polishing=True)])
+def test_cycles(kw):
+    lp, _ = G.random_lp(400, 1000, 4, 12, 8)
+    _same(lp, SELL, **kw)
+
+
+def test_repeated_solves_and_warm_start():
+    lp, _ = G.random_lp(300, 800, 4, 12, 9)
+    r, s = _solve(lp)
+    x, y = s.getPrimalValues(), s.getDualValues()
+    q = s.solve()
+    assert (q.iterations, q.objective) == (r.iterations, r.objective)
+    np.testing.assert_array_equal(s.getPrimalValues(), x)
+    s.setWarmStart(x, y)
+    w = s.solve()
+    _, t = _solve(lp, **SELL)
+    t.setWarmStart(x, y)
+    v = t.solve()
+    assert (w.iterations, w.objective) == (v.iterations, v.objective)
+    np.testing.assert_array_equal(s.getPrimalValues(), t.getPrimalValues())
+
+
+def test_many_threads():
+    """More waiting grids than the SMs hold: every solve ends with the bits it has alone."""
+    lp, _ = G.random_lp(2000, 5000, 4, 12, 5)
+    alone, s = _solve(lp)
+    out = [None] * 12
+
+    def go(k):
+        r, t = _solve(lp)
+        out[k] = (r.iterations, r.objective, t.getDualValues())
+
+    ts = [threading.Thread(target=go, args=(k,)) for k in range(len(out))]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    y = s.getDualValues()
+    for r in out:
+        assert r is not None and r[:2] == (alone.iterations, alone.objective)
+        np.testing.assert_array_equal(r[2], y)
