@@ -87,45 +87,104 @@ __global__ void __launch_bounds__(kBlock) controller(DevState* st, const DevCons
 }
 
 // ---- power iteration -------------------------------------------------------
-__global__ void __launch_bounds__(kBlock) powerFinish1(PowerArgs a) {
-    if (a.ps->done) return;
-    __shared__ double out[2];
-    const int ops[2] = {OP_SUM, OP_SUM};
-    reducePartials<2>(a.part, a.nb, ops, out);
+// Whether a chunk's iteration `it`, whose residual this is, ends the power
+// iteration.
+__device__ __forceinline__ bool powerEnds(const PowerArgs& a, int it, double resid) {
+    return a.ps->nrmv[it & 1] < 1e-15 || resid < a.tol * fabs(a.ps->s2v[it & 1]) || a.ps->iter + it + 1 >= a.max_iter;
+}
+
+// x = x_n / ||x_n|| of a chunk's iteration `it`, and its residual partials: nb
+// groups of kBlock threads' worth of columns, kNormGroups of them per block.
+// Every block sums the dot partials for itself, in their fixed order, and the
+// residual partials of the iteration before, which may have ended it all (its
+// products are then not used).  A single-block launch for either sum, 4.4 us and
+// a launch gap each, stood between the products before; one block elected by a
+// counter, the last to finish, was slower still (1,184 atomics on one word), and
+// so were four times fewer blocks of 1,024 threads.
+constexpr int kNormGroups = 4;
+__global__ void __launch_bounds__(kBlock) powerNormalize(PowerArgs a, int it) {
+    // read once per block: block 0 may set it while others start
+    __shared__ int done;
+    __shared__ double sums[3];
+    if (threadIdx.x == 0) done = a.ps->done;
+    const int t = static_cast<int>(threadIdx.x);
+    const bool check = it > 0;
+    {
+        const double* last = a.rpart + static_cast<size_t>((it - 1) & 1) * a.nb;
+        double acc[3] = {0.0, 0.0, 0.0};
+        for (int b = t; b < a.nb; b += kBlock) {
+            acc[0] += a.part[static_cast<size_t>(b) * 2];
+            acc[1] += a.part[static_cast<size_t>(b) * 2 + 1];
+            if (check) acc[2] += last[b];
+        }
+        const int ops[3] = {OP_SUM, OP_SUM, OP_SUM};
+        blockReduceSlots<3>(acc, ops, sums);
+    }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        a.ps->s2 = out[0];
-        a.ps->nrm = sqrt(out[1]);
+    if (done) return;
+    if (check) {
+        const double resid = sqrt(sums[2]);
+        if (powerEnds(a, it - 1, resid)) {
+            if (blockIdx.x == 0 && t == 0) {
+                a.ps->s2 = a.ps->s2v[(it - 1) & 1];
+                a.ps->resid = resid;
+                a.ps->done = 1;
+            }
+            return;
+        }
+    }
+    const double s2 = sums[0], nrm = sqrt(sums[1]);
+    const int g0 = static_cast<int>(blockIdx.x) * kNormGroups;
+    double acc[kNormGroups];
+#pragma unroll
+    for (int g = 0; g < kNormGroups; ++g) acc[g] = 0.0;
+    for (int64_t j0 = 0; j0 < a.n; j0 += static_cast<int64_t>(a.nb) * kBlock) {
+        double xn[kNormGroups], x[kNormGroups];
+#pragma unroll
+        for (int g = 0; g < kNormGroups; ++g) {
+            const int64_t j = j0 + (g0 + g) * kBlock + t;
+            const bool in = g0 + g < a.nb && j < a.n;
+            xn[g] = in ? a.xn[j] : 0.0;
+            x[g] = in ? a.x[j] : 0.0;
+        }
+#pragma unroll
+        for (int g = 0; g < kNormGroups; ++g) {
+            const int64_t j = j0 + (g0 + g) * kBlock + t;
+            if (g0 + g >= a.nb || j >= a.n) continue;
+            const double d = xn[g] - s2 * x[g];
+            acc[g] += d * d;
+            if (nrm >= 1e-15) a.x[j] = xn[g] / nrm;
+        }
+    }
+    const int ops[kNormGroups] = {OP_SUM, OP_SUM, OP_SUM, OP_SUM};
+    __shared__ double out[kNormGroups];
+    blockReduceSlots<kNormGroups>(acc, ops, out);
+    __syncthreads();
+    if (t < kNormGroups && g0 + t < a.nb) a.rpart[static_cast<size_t>(it & 1) * a.nb + g0 + t] = out[t];
+    if (blockIdx.x == 0 && t == 0) {
+        a.ps->s2v[it & 1] = s2;
+        a.ps->nrmv[it & 1] = nrm;
     }
 }
 
-__global__ void __launch_bounds__(kBlock) powerNormalize(PowerArgs a) {
-    if (a.ps->done) return;
-    const double s2 = a.ps->s2, nrm = a.ps->nrm;
-    double acc[1] = {0.0};
-    for (int j = blockIdx.x * kBlock + threadIdx.x; j < a.n; j += gridDim.x * kBlock) {
-        const double xn = a.xn[j];
-        const double d = xn - s2 * a.x[j];
-        acc[0] += d * d;
-        if (nrm >= 1e-15) a.x[j] = xn / nrm;
-    }
-    const int ops[1] = {OP_SUM};
-    blockReduceSlots<1>(acc, ops, a.part + static_cast<size_t>(blockIdx.x) * 2);
-}
-
-__global__ void __launch_bounds__(kBlock) powerFinish2(PowerArgs a) {
+// The end of a chunk of `its` iterations (an even number): the verdict on the
+// last one.
+__global__ void __launch_bounds__(kBlock) powerChunkEnd(PowerArgs a, int its) {
     if (a.ps->done) return;
     __shared__ double out[1];
-    double acc[1] = {0.0};
-    for (int b = threadIdx.x; b < a.nb; b += kBlock) acc[0] += a.part[static_cast<size_t>(b) * 2];
+    const double* part = a.rpart + static_cast<size_t>((its - 1) & 1) * a.nb;
     const int ops[1] = {OP_SUM};
+    double acc[1] = {0.0};
+    for (int b = threadIdx.x; b < a.nb; b += kBlock) acc[0] += part[b];
     blockReduceSlots<1>(acc, ops, out);
     __syncthreads();
     if (threadIdx.x == 0) {
-        PowerState& p = *a.ps;
-        p.resid = sqrt(out[0]);
-        p.iter += 1;
-        if (p.nrm < 1e-15 || p.resid < a.tol * fabs(p.s2) || p.iter >= a.max_iter) p.done = 1;
+        const double resid = sqrt(out[0]);
+        const bool ends = powerEnds(a, its - 1, resid);
+        a.ps->s2 = a.ps->s2v[(its - 1) & 1];
+        a.ps->resid = resid;
+        a.ps->iter += its;
+        a.ps->done = ends ? 1 : 0;
     }
 }
 
@@ -350,34 +409,52 @@ __global__ void __launch_bounds__(linkThreads(CSR), 1) linkedSteps(LinkArgs<T> a
 // per row, its entries summed in order in FP64, 8 per round.  On the
 // 500k x 2M power-law LP the CSR A^T launch (2 lanes per column) took 3.3x the
 // primal step's sliced-ELL time over the same columns.
-template <class V>
+template <int U, class V>
 __global__ void __launch_bounds__(kBlock) powerASell(PowerArgs a, const int2* __restrict__ hdr,
                                                     const int* __restrict__ idx, const V* __restrict__ val, int begin,
                                                     int end) {
-    if (a.ps->done) return;
     const int r = static_cast<int>(blockIdx.x) * kBlock + static_cast<int>(threadIdx.x);
-    if (begin + r >= end) return;
-    a.y[begin + r] = sellDot<8, V, double>(idx, val, hdr[r / kSlice], static_cast<int>(threadIdx.x) & 31, a.x);
+    const int2 h = hdr[min(r, end - begin - 1) / kSlice];
+    pdlWait();
+    pdlTrigger();
+    if (a.ps->done || begin + r >= end) return;
+    a.y[begin + r] = sellDot<U, V, double>(idx, val, h, static_cast<int>(threadIdx.x) & 31, a.x);
 }
 
-template <class V>
-__global__ void __launch_bounds__(kBlock) powerAtSell(PowerArgs a, const int2* __restrict__ hdr,
+// The short columns [begin, end) in sliced ELL, and in the first `lblocks`
+// blocks the long columns [0, begin) as CSR rows of G lanes: two launches in
+// one, so that neither trails off alone.  Bound by L1's tag stage, one scattered
+// sector per clock and SM: at 8 resident blocks (32 registers) 99 us on the
+// 500k x 2M power-law LP against 84 + 51 us apart (20.1M gathers are 69 us).
+// With the sums in powerNormalize an iteration there went from 250 to 211 us.
+template <int G, int U, class V>
+__global__ void __launch_bounds__(kBlock, sizeof(V) == 4 ? 8 : 4) powerAtSell(PowerArgs a, PowerMat<V> mt, const int2* __restrict__ hdr,
                                                      const int* __restrict__ idx, const V* __restrict__ val, int begin,
-                                                     int end, int part0) {
+                                                     int end, int lblocks) {
+    pdlWait();
+    pdlTrigger();
     if (a.ps->done) return;
     double acc[2] = {0.0, 0.0};
-    const int rows = end - begin;
-    // the stride is a multiple of 32, so a thread keeps its lane of every slice
-    for (int r = static_cast<int>(blockIdx.x) * kBlock + static_cast<int>(threadIdx.x); r < rows;
-         r += static_cast<int>(gridDim.x) * kBlock) {
-        const int j = begin + r;
-        const double s = sellDot<8, V, double>(idx, val, hdr[r / kSlice], static_cast<int>(threadIdx.x) & 31, a.y);
-        a.xn[j] = s;
-        acc[0] += a.x[j] * s;
-        acc[1] += s * s;
+    const int sblocks = static_cast<int>(gridDim.x) - lblocks;
+    int b = static_cast<int>(blockIdx.x);
+    int part;
+    if (b < lblocks) {
+        powerAtRows<G, V>(a, mt, 0, begin, b, lblocks, acc);
+        part = sblocks + b;
+    } else {
+        part = b -= lblocks;
+        const int rows = end - begin;
+        // the stride is a multiple of 32, so a thread keeps its lane of every slice
+        for (int r = b * kBlock + static_cast<int>(threadIdx.x); r < rows; r += sblocks * kBlock) {
+            const int j = begin + r;
+            const double s =
+                sellDot<U, V, double>(idx, val, hdr[r / kSlice], static_cast<int>(threadIdx.x) & 31, a.y);
+            a.xn[j] = s;
+            acc[0] += a.x[j] * s;
+            acc[1] += s * s;
+        }
     }
-    const int ops[2] = {OP_SUM, OP_SUM};
-    blockReduceSlots<2>(acc, ops, a.part + static_cast<size_t>(part0 + blockIdx.x) * 2);
+    powerAtEnd(a, acc, part);
 }
 
 // Sliced-ELL shapes of the single-LP engine: kNumShapes + k for k < kEngSell,
@@ -489,7 +566,7 @@ struct DeviceLp {
     double *yc64 = nullptr, *yi64 = nullptr, *yh64 = nullptr;
     float* yg32 = nullptr;  // FP32 copy of yc, gathered by the mixed-mode primal step
     double *prev_ax = nullptr, *prev_xh = nullptr;
-    double *pi_x = nullptr, *pi_y = nullptr, *pi_xn = nullptr, *pi_part = nullptr;
+    double *pi_x = nullptr, *pi_y = nullptr, *pi_xn = nullptr, *pi_part = nullptr, *pi_rpart = nullptr;
     double *part_rows = nullptr, *part_cols = nullptr;
     // Anderson acceleration at restarts (anderson.cuh); aa_w = 0 when off.
     int aa_w = 0, aa_nb = 1;
@@ -516,7 +593,7 @@ struct DeviceLp {
     cudaGraphExec_t power = nullptr;
     int launches_cycle[2][2] = {{0, 0}, {0, 0}};
     int launches_power = 0;
-    static constexpr int kPowerChunk = 8;
+    static constexpr int kPowerChunk = 8;  // even (powerChunkEnd)
 
     ~DeviceLp() {
         for (auto& row : cycle)
@@ -1026,31 +1103,36 @@ template <class V>
 int launchPowerChunk(DeviceLp& d, const PowerArgs& pa, const PowerMat<V>& mt, int chunk) {
     cudaStream_t s = d.stream;
     int launches = 0;
+    const double meanP = static_cast<double>(d.nnz - d.zlP) / std::max(1, d.n - d.nlP);
+    const double meanD = static_cast<double>(d.nnz - d.zlD) / std::max(1, d.m - d.nlD);
     for (int it = 0; it < chunk; ++it) {
         // A x for every row before A^T y reads it
         if (isSell(d.shapeD))
-            powerASell<V><<<sellGrid(d.m - d.nlD), kBlock, 0, s>>>(pa, d.sd_hdr, d.sd_idx, sellVals<V>(d, false),
-                                                                   d.nlD, d.m);
+            launchPdl(meanD <= 12.0 ? powerASell<4, V> : powerASell<8, V>, sellGrid(d.m - d.nlD), kBlock, 0, s, pa,
+                      d.sd_hdr, d.sd_idx, sellVals<V>(d, false), d.nlD, d.m);
         else
             PDLPX_G_SWITCH(d.gA, (powerA<GG, V><<<gridFor(d.m - d.nlD, d.gA), kBlock, 0, s>>>(pa, mt, d.nlD, d.m)));
         if (d.nlD > 0) {
             PDLPX_G_SWITCH(d.gLA, (powerA<GG, V><<<gridFor(d.nlD, d.gLA), kBlock, 0, s>>>(pa, mt, 0, d.nlD)));
             ++launches;
         }
-        if (isSell(d.shapeP))
-            powerAtSell<V><<<d.nb_pi_s, kBlock, 0, s>>>(pa, d.sp_hdr, d.sp_idx, sellVals<V>(d, true), d.nlP, d.n, 0);
-        else
+        const int lblocks = d.nb_pi - d.nb_pi_s;
+        if (isSell(d.shapeP)) {
+            PDLPX_G_SWITCH(d.gLAT, launchPdl(meanP <= 12.0 ? powerAtSell<GG, 4, V> : powerAtSell<GG, 8, V>, d.nb_pi,
+                                             kBlock, 0, s, pa, mt, d.sp_hdr, d.sp_idx, sellVals<V>(d, true), d.nlP,
+                                             d.n, lblocks));
+        } else {
             PDLPX_G_SWITCH(d.gAT, (powerAt<GG, V><<<d.nb_pi_s, kBlock, 0, s>>>(pa, mt, d.nlP, d.n, 0)));
-        if (d.nlP > 0) {
-            PDLPX_G_SWITCH(d.gLAT, (powerAt<GG, V><<<d.nb_pi - d.nb_pi_s, kBlock, 0, s>>>(pa, mt, 0, d.nlP, d.nb_pi_s)));
-            ++launches;
+            if (d.nlP > 0) {
+                PDLPX_G_SWITCH(d.gLAT, (powerAt<GG, V><<<lblocks, kBlock, 0, s>>>(pa, mt, 0, d.nlP, d.nb_pi_s)));
+                ++launches;
+            }
         }
-        powerFinish1<<<1, kBlock, 0, s>>>(pa);
-        powerNormalize<<<d.nb_pi, kBlock, 0, s>>>(pa);
-        powerFinish2<<<1, kBlock, 0, s>>>(pa);
-        launches += 5;
+        powerNormalize<<<(d.nb_pi + kNormGroups - 1) / kNormGroups, kBlock, 0, s>>>(pa, it);
+        launches += 3;
     }
-    return launches;
+    powerChunkEnd<<<1, kBlock, 0, s>>>(pa, chunk);
+    return launches + 1;
 }
 
 template <class T>
@@ -1502,7 +1584,7 @@ static int32_t buildDevice(std::unique_ptr<DeviceLp>& dp, const ScaledLp& sc_in,
     const bool adaptive = o.adaptive_step != 0;
     const size_t o_prev_ax = adaptive ? take(8 * m) : 0, o_prev_xh = adaptive ? take(8 * n) : 0;
     const size_t o_pi_x = take(8 * n), o_pi_y = take(8 * m), o_pi_xn = take(8 * n),
-                 o_pi_part = take(8 * 2 * d.nb_pi);
+                 o_pi_part = take(8 * 4 * d.nb_pi);  // dot partials, residual partials by parity
     // cells of the linked cycle
     const bool link = linkable(d, o);
     const size_t o_lx = link ? take(sizeof(LinkCell<double>) * n) : 0, o_ly = link ? take(sizeof(LinkCell<double>) * m) : 0;
@@ -1586,6 +1668,7 @@ static int32_t buildDevice(std::unique_ptr<DeviceLp>& dp, const ScaledLp& sc_in,
     d.pi_y = reinterpret_cast<double*>(b + o_pi_y);
     d.pi_xn = reinterpret_cast<double*>(b + o_pi_xn);
     d.pi_part = reinterpret_cast<double*>(b + o_pi_part);
+    d.pi_rpart = d.pi_part + 2 * static_cast<size_t>(d.nb_pi);
     d.part_rows = reinterpret_cast<double*>(b + o_prow);
     d.part_cols = reinterpret_cast<double*>(b + o_pcol);
     if (sellP) {
@@ -2120,6 +2203,7 @@ int32_t Engine::solveDevice(pdlpx_result* out) {
         pa.xn = d.pi_xn;
         pa.part = d.pi_part;
         pa.ps = d.ps;
+        pa.rpart = d.pi_rpart;
         pa.m = m;
         pa.n = n;
         pa.max_iter = opt_.sv_max_iter;

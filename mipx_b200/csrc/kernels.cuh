@@ -996,6 +996,8 @@ struct PowerState {
     double resid; // ||A^T A x - s2 x||
     int iter;
     int done;
+    // s2 and nrm of the single-LP engine's last two iterations, by parity
+    double s2v[2], nrmv[2];
 };
 struct PowerArgs {
     double* x;
@@ -1003,6 +1005,7 @@ struct PowerArgs {
     double* xn;
     double* part;  // [nb][2]
     PowerState* ps;
+    double* rpart;  // [2][nb] residual partials, by the iteration's parity
     int m, n, max_iter, nb;
     double tol;
 };
@@ -1026,13 +1029,13 @@ __global__ void __launch_bounds__(kBlock) powerA(PowerArgs a, PowerMat<V> mt, in
     s = groupSum<G>(s);
     if (valid && lane == 0) a.y[i] = s;
 }
+// Rows [begin, end) of A^T by `blocks` blocks, this one the b-th.
 template <int G, class V>
-__global__ void __launch_bounds__(kBlock) powerAt(PowerArgs a, PowerMat<V> mt, int begin, int end, int part0) {
-    if (a.ps->done) return;
-    const int per_block = kBlock / G;
+__device__ __forceinline__ void powerAtRows(const PowerArgs& a, const PowerMat<V>& mt, int begin, int end, int b,
+                                            int blocks, double (&acc)[2]) {
+    constexpr int per_block = kBlock / G;
     const int lane = threadIdx.x % G;
-    double acc[2] = {0.0, 0.0};
-    for (int base = begin + static_cast<int>(blockIdx.x) * per_block; base < end; base += gridDim.x * per_block) {
+    for (int base = begin + b * per_block; base < end; base += blocks * per_block) {
         const int j = base + threadIdx.x / G;
         const bool valid = j < end;
         double s = 0.0;
@@ -1044,12 +1047,18 @@ __global__ void __launch_bounds__(kBlock) powerAt(PowerArgs a, PowerMat<V> mt, i
             acc[1] += s * s;
         }
     }
-    const int ops[2] = {OP_SUM, OP_SUM};
-    blockReduceSlots<2>(acc, ops, a.part + static_cast<size_t>(part0 + blockIdx.x) * 2);
 }
-__global__ void powerFinish1(PowerArgs a);
-__global__ void __launch_bounds__(kBlock) powerNormalize(PowerArgs a);
-__global__ void powerFinish2(PowerArgs a);
+__device__ __forceinline__ void powerAtEnd(const PowerArgs& a, double (&acc)[2], int part) {
+    const int ops[2] = {OP_SUM, OP_SUM};
+    blockReduceSlots<2>(acc, ops, a.part + static_cast<size_t>(part) * 2);
+}
+template <int G, class V>
+__global__ void __launch_bounds__(kBlock) powerAt(PowerArgs a, PowerMat<V> mt, int begin, int end, int part0) {
+    if (a.ps->done) return;
+    double acc[2] = {0.0, 0.0};
+    powerAtRows<G, V>(a, mt, begin, end, static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x), acc);
+    powerAtEnd(a, acc, part0 + static_cast<int>(blockIdx.x));
+}
 
 // Plain SpMV for the parity entry point pdlpx_csr_spmv (FP64 accumulation, like the step kernels).
 template <int G, class T>
