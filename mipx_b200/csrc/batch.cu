@@ -27,7 +27,9 @@
 // pack -- N iterations, the FP64 check, the controllers, restart copies, FP32
 // -> FP64 hand-overs and the tile modes -- is one CUDA graph launch.  When
 // finished LPs leave enough tiles idle, the host switches the launches to a
-// list of the live tiles and captures a smaller graph.
+// list of the live tiles and captures a smaller graph.  While the live LPs of a
+// sliced-ELL pack are few (kLinkPackEntries) their steps run as one linked cycle
+// instead (linked.cuh), with the same bits.
 //
 // An LP's tiles, launch shape, storage and reduction order depend on that LP
 // alone, so its result is bit-identical alone and in any mix (batch
@@ -49,6 +51,7 @@
 #include "control.cuh"
 #include "engine.hpp"
 #include "kernels.cuh"
+#include "linked.cuh"
 #include "pack.hpp"
 #include "shapes.cuh"
 
@@ -300,6 +303,143 @@ __global__ void __launch_bounds__(kBlock, PDLPX_SELL_MIN_BLOCKS) packCycleSell(P
                 dualSellTile<kSellU[1]>(a, e.x, e.y + t, k);
         }
         if (!gridBarrier(q.bar, q.err)) return;
+    }
+}
+
+// ---- linked cycle (linked.cuh) of a pack of sliced-ELL LPs ----------------------
+// The live LPs' rows and columns as one list of units, a warp's work each: every
+// LP runs at its own pace, in its own precision.  Cells: x_refl as FP32 or FP64
+// (of the LP's precision), y as FP64, as the step kernels gather it.
+struct LinkLp {  // of one LP for the cycle at hand
+    double step, pw;
+    int inner, iters;  // iters 0: the LP is done
+    unsigned base;     // number of the cycle's first y
+    int prec;
+};
+struct LinkPackArgs {
+    const int4* punits;  // (LP, first column, end column, slice)
+    const int4* dunits;  // (LP, first row, end row, slice)
+    LinkLp* lp;
+    LinkCell<float>* xf;
+    LinkCell<double>* xd;
+    LinkCell<double>* y;
+    int* err;
+    int np, nd, N;
+};
+constexpr int kLinkPackThreads = 512;
+// Live entries up to which the linked cycle runs a pack's steps.  Measured on
+// B200 (ms per batch_solve, launches -> linked): 12 LPs of 118k entries in FP64
+// 187 -> 88, 6 of 454k 69 -> 56; 64 LPs of 2.1M entries 280 with launches, 362
+// linked throughout, and 254 linked once the live LPs are down to 1M (266 from
+// 400k on).
+constexpr int64_t kLinkPackEntries = 1000000;
+
+__global__ void packLinkBegin(PackArgs a, LinkPackArgs q) {
+    const int l = blockIdx.x * blockDim.x + threadIdx.x;
+    if (l >= a.L) return;
+    const DevState& s = a.st[l];
+    const int cur = s.phase == 0 ? s.total : s.polish_count;
+    const int lim = s.phase == 0 ? a.it64.max_iter : a.it64.polish_max_iter;
+    q.lp[l] = LinkLp{s.step,
+                     s.pw,
+                     s.inner,
+                     s.done ? 0 : max(0, min(q.N, lim - cur)),
+                     static_cast<unsigned>(s.checks) * static_cast<unsigned>(q.N + 1) + 1u,
+                     s.prec};
+}
+
+// Column j (-1: none) of a unit, its sum by gathers of y, its step.
+template <int L, class T>
+__device__ __forceinline__ void linkPackPrimal(const IterArgs<T>& p, const int* idx, const T* val, int2 h, int r,
+                                               int lane, int j, const LinkLp& lp, int it, double lam,
+                                               const LinkCell<double>* y, LinkCell<T>* x, int* err, bool& ok) {
+    ColPack<T> c{};
+    double xcd = 0.0, xi = 0.0, tau = 0.0;
+    if (j >= 0) {
+        c = p.cp[j];
+        xcd = p.xc[j];
+        xi = static_cast<double>(p.xi[j]);
+        tau = lp.step * static_cast<double>(c.tau) / lp.pw;
+    }
+    const unsigned tag = lp.base + static_cast<unsigned>(it);
+    const double s = linkSellDot<L>(idx, val, h, r, lane, y, tag - 1u, err, ok);
+    if (j < 0) return;
+    double xh, xr;
+    const double xn = primalValues<T>(c, xcd, xi, s, tau, lam, xh, xr);
+    linkStore(x + j, static_cast<T>(xr), tag);
+    p.xc[j] = xn;
+    if (it == lp.iters) p.xh[j] = static_cast<T>(xh);
+}
+template <int L, class T>
+__device__ __forceinline__ void linkPackDual(const IterArgs<T>& p, const int* idx, const T* val, int2 h, int r,
+                                             int lane, int i, const LinkLp& lp, int it, double lam,
+                                             const LinkCell<T>* x, LinkCell<double>* y, int* err, bool& ok) {
+    RowPack<T> c{};
+    double ycd = 0.0, yi = 0.0;
+    if (i >= 0) {
+        c = p.rp[i];
+        ycd = p.yc[i];
+        yi = static_cast<double>(p.yi[i]);
+    }
+    const unsigned tag = lp.base + static_cast<unsigned>(it);
+    const double s = linkSellDot<L>(idx, val, h, r, lane, x, tag, err, ok);
+    if (i < 0) return;
+    double py;
+    const double yn = dualValues<T>(c, ycd, yi, s, lp.step, lp.pw, lam, py);
+    linkStore(y + i, yn, tag);
+    p.yc[i] = yn;
+    if (it == lp.iters) p.yh[i] = static_cast<T>(py);
+}
+
+// LP / LD: lanes per column / row.
+template <int LP, int LD>
+__global__ void __launch_bounds__(kLinkPackThreads, 1) packLinked(PackArgs a, LinkPackArgs q) {
+    const int lane = static_cast<int>(threadIdx.x) & 31;
+    const int wid = static_cast<int>(blockIdx.x) + static_cast<int>(gridDim.x) * (static_cast<int>(threadIdx.x) >> 5);
+    const int nw = static_cast<int>(gridDim.x) * (static_cast<int>(blockDim.x) >> 5);
+    const int firstD = ((wid - q.np) % nw + nw) % nw;
+    // row of this lane, and its place in the slice
+    auto rowOf = [&](const int4& u, int L) {
+        const int r = u.y + lane / L;
+        return r < u.z && lane % L == 0 ? r : -1;
+    };
+    for (int u = firstD; u < q.nd; u += nw) {
+        const int4 d = __ldg(q.dunits + u);
+        const LinkLp lp = q.lp[d.x];
+        const int i = rowOf(d, LD);
+        if (lp.iters > 0 && i >= 0) linkStore(q.y + i, a.it64.yc[i], lp.base);
+    }
+    bool ok = true;
+    for (int it = 1; it <= q.N; ++it) {
+        for (int u = wid; u < q.np; u += nw) {
+            const int4 d = __ldg(q.punits + u);
+            const LinkLp lp = q.lp[d.x];
+            if (it > lp.iters) continue;
+            const int k = lp.inner + it;
+            const double lam = static_cast<double>(k) / static_cast<double>(k + 1);
+            const int j = rowOf(d, LP), r = (d.y & 31) + lane / LP;
+            const int2 h = __ldg(a.cs.hdr + d.w);
+            if (lp.prec == 0)
+                linkPackPrimal<LP, float>(a.it32, a.cs.idx, a.cs.v32, h, r, lane, j, lp, it, lam, q.y, q.xf, q.err, ok);
+            else
+                linkPackPrimal<LP, double>(a.it64, a.cs.idx, a.cs.v64, h, r, lane, j, lp, it, lam, q.y, q.xd, q.err, ok);
+        }
+        __syncwarp();
+        for (int u = firstD; u < q.nd; u += nw) {
+            const int4 d = __ldg(q.dunits + u);
+            const LinkLp lp = q.lp[d.x];
+            if (it > lp.iters) continue;
+            const int k = lp.inner + it;
+            const double lam = static_cast<double>(k) / static_cast<double>(k + 1);
+            const int i = rowOf(d, LD), r = (d.y & 31) + lane / LD;
+            const int2 h = __ldg(a.rs.hdr + d.w);
+            if (lp.prec == 0)
+                linkPackDual<LD, float>(a.it32, a.rs.idx, a.rs.v32, h, r, lane, i, lp, it, lam, q.xf, q.y, q.err, ok);
+            else
+                linkPackDual<LD, double>(a.it64, a.rs.idx, a.rs.v64, h, r, lane, i, lp, it, lam, q.xd, q.y, q.err, ok);
+        }
+        __syncwarp();
+        if (__any_sync(0xffffffffu, !ok)) return;
     }
 }
 
@@ -615,6 +755,7 @@ size_t itemBytes(const Item& it, bool mixed) {
     b += static_cast<size_t>(it.cols.entries + it.rows.entries) * (4 + 8 + (mixed ? 4 : 0)) + (m + n) / 4;
     b += static_cast<size_t>(it.nct) * (16 + 4 + 8 * kColSlots + 16) + static_cast<size_t>(it.nrt) * (16 + 4 + 8 * kRowSlots);
     b += sizeof(DevState) + sizeof(DevConst) + sizeof(PowerState) + 32;
+    b += n * (16 + 2 + (mixed ? 8 : 0)) + m * (16 + 4) + sizeof(LinkLp);  // linked cycle: cells, units
     return b;
 }
 
@@ -711,6 +852,14 @@ struct Pack {
     int live_ct = 0, live_rt = 0;      // tiles in the current launches
     std::vector<int> h_cl, h_rl;       // host copies of the live-tile lists
     PackArgs args{};
+    // linked cycle: cells and unit lists of the live LPs
+    bool linkable = false;       // every side is sliced ELL
+    bool linked = false;         // the live LPs are few enough
+    int link_lanes = 4, link_warps = 0;
+    cudaGraphExec_t lcycle = nullptr;
+    int lcycle_launches = 0;
+    std::vector<int4> h_pu, h_du;
+    size_t o_pu = 0, o_du = 0, o_lp = 0, o_lxf = 0, o_lxd = 0, o_ly = 0;
     // persistent cycle (option batch_persistent): tile lists, barrier words
     // [arrivals, generation, error, -], cooperative grid
     bool persist = false;
@@ -722,6 +871,7 @@ struct Pack {
     // other packs run, and a plain free would wait for the whole device.
     ~Pack() {
         if (cycle) cudaGraphExecDestroy(cycle);
+        if (lcycle) cudaGraphExecDestroy(lcycle);
         if (power) cudaGraphExecDestroy(power);
         if (pd) cudaFreeAsync(pd, s);
         if (d) cudaFreeAsync(d, s);
@@ -783,6 +933,8 @@ struct Pack {
         listed = false;
         live_ct = nct;
         live_rt = nrt;
+        linkable = true;
+        for (const Item* it : items) linkable = linkable && isSell(it->shapeP) && isSell(it->shapeD);
     }
 
     void layout() {
@@ -850,8 +1002,21 @@ struct Pack {
         o_prows = take(8 * kRowSlots * static_cast<size_t>(nrt));
         o_clist = take(4 * static_cast<size_t>(nct));
         o_rlist = take(4 * static_cast<size_t>(nrt));
-        o_flags = take(4 * static_cast<size_t>(L));
+        o_flags = take(4 * (static_cast<size_t>(L) + 1));  // the linked cycle's error word last
         o_counters = take(64);
+        if (linkable) {
+            size_t pu = 0, du = 0;
+            for (const Item* it : items) {
+                pu += (static_cast<size_t>(it->lp.n) + 7) / 8;
+                du += (static_cast<size_t>(it->lp.m) + 3) / 4;
+            }
+            o_pu = take(sizeof(int4) * pu);
+            o_du = take(sizeof(int4) * du);
+            o_lp = take(sizeof(LinkLp) * L);
+            o_lxf = mixed ? take(sizeof(LinkCell<float>) * n) : 0;
+            o_lxd = take(sizeof(LinkCell<double>) * n);
+            o_ly = take(sizeof(LinkCell<double>) * m);
+        }
         total = o;
     }
 
@@ -1007,6 +1172,69 @@ struct Pack {
             e = cudaMemcpyAsync(pd + 16 + sizeof(int4) * static_cast<size_t>(nct), h_dtiles.data(),
                                 sizeof(int4) * h_dtiles.size(), cudaMemcpyHostToDevice, s);
         return e;
+    }
+
+    // Whether the linked cycle runs the LPs with keep[l] set, and its unit lists,
+    // uploaded on the pack's stream.
+    cudaError_t planLinked(const std::vector<char>& keep, int sms) {
+        linked = false;
+        link_warps = 0;
+        if (!linkable) return cudaSuccess;
+        int64_t z = 0, units = 0;
+        for (const Item* it : items)
+            if (keep[it->l]) {
+                z += it->sc.a.nnz();
+                units += (it->lp.n + 7) / 8 + (it->lp.m + 3) / 4;
+            }
+        if (z > kLinkPackEntries || units == 0) return cudaSuccess;
+        const int warps_max = kLinkPackThreads / 32;
+        link_lanes = units <= 3 * static_cast<int64_t>(sms) * warps_max ? 4 : 2;
+        const int rc = kSlice / link_lanes, rr = kSlice / (2 * link_lanes);
+        h_pu.clear();
+        h_du.clear();
+        for (const Item* it : items) {
+            if (!keep[it->l]) continue;
+            const int c0 = static_cast<int>(it->c0), r0 = static_cast<int>(it->r0);
+            for (int j = 0; j < it->lp.n; j += rc) h_pu.push_back(make_int4(it->l, c0 + j, c0 + it->lp.n, (c0 + j) / kSlice));
+            for (int i = 0; i < it->lp.m; i += rr) h_du.push_back(make_int4(it->l, r0 + i, r0 + it->lp.m, (r0 + i) / kSlice));
+        }
+        const int64_t total_units = static_cast<int64_t>(h_pu.size() + h_du.size());
+        link_warps = static_cast<int>(std::min<int64_t>(warps_max, (total_units + sms - 1) / sms));
+        linked = true;
+        cudaError_t e = cudaMemcpyAsync(d + o_pu, h_pu.data(), sizeof(int4) * h_pu.size(), cudaMemcpyHostToDevice, s);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(d + o_du, h_du.data(), sizeof(int4) * h_du.size(), cudaMemcpyHostToDevice, s);
+        return e;
+    }
+
+    // The steps of one cycle over the planned units.
+    int launchLinked(int N, int sms) {
+        LinkPackArgs q{P<int4>(o_pu),
+                       P<int4>(o_du),
+                       P<LinkLp>(o_lp),
+                       mixed ? P<LinkCell<float>>(o_lxf) : nullptr,
+                       P<LinkCell<double>>(o_lxd),
+                       P<LinkCell<double>>(o_ly),
+                       P<int>(o_flags) + L,
+                       static_cast<int>(h_pu.size()),
+                       static_cast<int>(h_du.size()),
+                       N};
+        packLinkBegin<<<(L + 127) / 128, 128, 0, s>>>(args, q);
+        const int units = q.np + q.nd;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(static_cast<unsigned>(std::min(sms, (units + link_warps - 1) / link_warps)));
+        cfg.blockDim = dim3(static_cast<unsigned>(32 * link_warps));
+        cfg.stream = s;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeCooperative;
+        at[0].val.cooperative = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        if (link_lanes == 4)
+            cudaLaunchKernelEx(&cfg, packLinked<4, 8>, args, q);
+        else
+            cudaLaunchKernelEx(&cfg, packLinked<2, 4>, args, q);
+        return 2;
     }
 
     // One persistent cycle of N iterations (barrier words cleared first).
@@ -1485,9 +1713,12 @@ int32_t solvePack(Pack& pk, const pdlpx_options& o, std::chrono::steady_clock::t
 
     // counters[0] / per-LP flags (pageable: a pinned allocation would
     // synchronize the device, which other packs share)
-    std::vector<int> h_flags(std::max(L, 16));
+    std::vector<int> h_flags(std::max(L + 1, 16));
     int* h_small = h_flags.data();
 
+    int dev = 0, sms = 0;
+    PDLPX_BCK(cudaGetDevice(&dev));
+    PDLPX_BCK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     auto capture = [&](cudaGraphExec_t& g, int& count, bool power) -> int32_t {
         if (g) {
             cudaGraphExecDestroy(g);
@@ -1495,7 +1726,12 @@ int32_t solvePack(Pack& pk, const pdlpx_options& o, std::chrono::steady_clock::t
         }
         cudaGraph_t graph = nullptr;
         PDLPX_BCK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-        count = power ? pk.launchPower(8) : pk.launchCycle(o.termination_eval_frequency, !pk.persist);
+        if (power)
+            count = pk.launchPower(8);
+        else if (&g == &pk.lcycle)
+            count = pk.launchLinked(o.termination_eval_frequency, sms) + pk.launchCycle(o.termination_eval_frequency, false);
+        else
+            count = pk.launchCycle(o.termination_eval_frequency, !pk.persist);
         PDLPX_BCK(cudaStreamEndCapture(s, &graph));
         const cudaError_t ie = cudaGraphInstantiate(&g, graph, 0);
         cudaGraphDestroy(graph);
@@ -1584,10 +1820,8 @@ int32_t solvePack(Pack& pk, const pdlpx_options& o, std::chrono::steady_clock::t
     // one cooperative launch ahead of the graph of its check, controller and
     // restart launches
     if (o.batch_persistent && pk.persistable()) {
-        int nb = 0, dev = 0, sms = 0, coop = 0;
+        int nb = 0, coop = 0;
         PDLPX_BCK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, packCycleSell, kBlock, 0));
-        PDLPX_BCK(cudaGetDevice(&dev));
-        PDLPX_BCK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         PDLPX_BCK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
         if (nb > 0 && coop) {
             pk.persist_grid = std::max(1, std::min(nb * sms, std::max(pk.nct, pk.nrt)));
@@ -1599,13 +1833,11 @@ int32_t solvePack(Pack& pk, const pdlpx_options& o, std::chrono::steady_clock::t
     }
 
     // ---- restart cycles; finished LPs are read back after the cycle that ends them
-    {
-        int32_t rc = capture(pk.cycle, pk.cycle_launches, false);
-        if (rc != PDLPX_OK) return rc;
-    }
+    std::vector<char> keep(L, 1), collected(L, 0);
+    if (!pk.persist) PDLPX_BCK(pk.planLinked(keep, sms));
+    LinkShare share(dev, pk.link_warps);
     int perr = 0;
     SleepWait sleeper;
-    std::vector<char> keep(L, 1), collected(L, 0);
     std::vector<int> cl, rl;
     int cycles = 0, ncollected = 0;
     while (ncollected < L) {
@@ -1614,15 +1846,26 @@ int32_t solvePack(Pack& pk, const pdlpx_options& o, std::chrono::steady_clock::t
             PDLPX_BCK(pk.launchPersistent(o.termination_eval_frequency));
             ++launches;
         }
-        PDLPX_BCK(cudaGraphLaunch(pk.cycle, s));
-        launches += pk.cycle_launches;
+        const bool linked = pk.linked && share.fits();
+        cudaGraphExec_t& graph = linked ? pk.lcycle : pk.cycle;
+        int& graph_launches = linked ? pk.lcycle_launches : pk.cycle_launches;
+        if (!graph) {
+            const int32_t rc = capture(graph, graph_launches, false);
+            if (rc != PDLPX_OK) return rc;
+        }
+        PDLPX_BCK(cudaGraphLaunch(graph, s));
+        launches += graph_launches;
         ++cycles;
         PDLPX_BCK(sleeper.wait(s));
-        PDLPX_BCK(cudaMemcpyAsync(h_small, pk.args.flags, 4 * static_cast<size_t>(L), cudaMemcpyDeviceToHost, s));
+        PDLPX_BCK(cudaMemcpyAsync(h_small, pk.args.flags, 4 * (static_cast<size_t>(L) + 1), cudaMemcpyDeviceToHost, s));
         if (pk.persist) PDLPX_BCK(cudaMemcpyAsync(&perr, pk.pd + 8, 4, cudaMemcpyDeviceToHost, s));
         PDLPX_BCK(cudaStreamSynchronize(s));
         if (perr != 0) {
             err = "persistent cycle: a grid barrier ran out of polls";
+            return PDLPX_E_TIMEOUT;
+        }
+        if (h_small[L] != 0) {
+            err = "linked cycle: a wait ran out of polls";
             return PDLPX_E_TIMEOUT;
         }
         int done_count = 0, fp64 = 0, live_tiles = 0;
@@ -1651,16 +1894,25 @@ int32_t solvePack(Pack& pk, const pdlpx_options& o, std::chrono::steady_clock::t
             std::fflush(stdout);
         }
         if (done_count >= L) break;
-        if (o.batch_compact && live_tiles < ((pk.live_ct + pk.live_rt) * 3) / 5) {
+        // a linked cycle's warps divide the live units between them, and its graph
+        // is small: it follows the live LPs more closely
+        const int64_t tiles = pk.live_ct + pk.live_rt;
+        if (o.batch_compact && live_tiles < (linked ? tiles * 9 / 10 : tiles * 3 / 5)) {
             for (int l = 0; l < L; ++l) keep[l] = !(h_small[l] & 1);
             pk.liveLists(keep, cl, rl);
             if (!cl.empty())
                 PDLPX_BCK(cudaMemcpyAsync(pk.d + pk.o_clist, cl.data(), 4 * cl.size(), cudaMemcpyHostToDevice, s));
             if (!rl.empty())
                 PDLPX_BCK(cudaMemcpyAsync(pk.d + pk.o_rlist, rl.data(), 4 * rl.size(), cudaMemcpyHostToDevice, s));
-            if (pk.persist) PDLPX_BCK(pk.uploadPersistTiles());
-            int32_t rc = capture(pk.cycle, pk.cycle_launches, false);
-            if (rc != PDLPX_OK) return rc;
+            if (pk.persist)
+                PDLPX_BCK(pk.uploadPersistTiles());
+            else
+                PDLPX_BCK(pk.planLinked(keep, sms));
+            share.set(pk.link_warps);
+            for (cudaGraphExec_t* g : {&pk.cycle, &pk.lcycle}) {
+                if (*g) cudaGraphExecDestroy(*g);
+                *g = nullptr;
+            }
         }
     }
     // LPs the time limit or the stop request left unfinished

@@ -970,31 +970,6 @@ void planLinked(DeviceLp& d) {
     d.link_warps = std::min(linkThreads(csr) / 32, (units + d.sms - 1) / d.sms);
 }
 
-// Warps per SM of the linked grids that the solves running on a device would
-// launch, by device.  Above kLinkShare of them a cycle runs by launches, which
-// share the SMs better than waiting grids do (16 solver threads on one B200, us
-// per LP-iteration of all: 2,000 x 5,000 launches 0.80, linked 2.05; with 4
-// threads 2.44 and 2.15).  Both give the same bits, so the choice is made anew
-// for every cycle.
-constexpr int kLinkShare = 32;
-std::atomic<int> g_link_warps[64];
-struct LinkShare {
-    std::atomic<int>* total = nullptr;
-    int warps = 0;
-    LinkShare(int device, int w) {
-        if (w <= 0 || device < 0 || device >= 64) return;
-        total = &g_link_warps[device];
-        warps = w;
-        total->fetch_add(warps, std::memory_order_relaxed);
-    }
-    ~LinkShare() {
-        if (total) total->fetch_sub(warps, std::memory_order_relaxed);
-    }
-    LinkShare(const LinkShare&) = delete;
-    LinkShare& operator=(const LinkShare&) = delete;
-    bool fits() const { return total != nullptr && total->load(std::memory_order_relaxed) <= std::max(kLinkShare, warps); }
-};
-
 template <int LP, int LD, bool CSR, class T>
 cudaError_t launchLinkedAs(const DeviceLp& d, LinkArgs<T>& a, cudaStream_t s) {
     a.P.units = linkUnits(a.P.rows, a.P.nl, a.P.lanes, LP);

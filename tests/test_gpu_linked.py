@@ -11,7 +11,7 @@ import numpy as np
 import pytest
 
 from mipx_b200 import generators as G
-from mipx_b200.pdlp import LpProblem, PdlpOptions, PdlpSolver, Precision, SparseMatrix
+from mipx_b200.pdlp import LpProblem, PdlpOptions, PdlpSolver, Precision, SparseMatrix, batch_solve
 
 pytestmark = pytest.mark.gpu
 
@@ -137,3 +137,39 @@ def test_many_threads():
     for r in out:
         assert r is not None and r[:2] == (alone.iterations, alone.objective)
         np.testing.assert_array_equal(r[2], y)
+
+
+# packs: the persistent cycle runs the step kernels' own tile functions
+@pytest.mark.parametrize("kw", [dict(), dict(precision=Precision.FP64), dict(max_iter=777), dict(batch_compact=False),
+                                dict(termination_eval_frequency=7, max_iter=300),
+                                dict(primal_tol=1e-6, dual_tol=1e-6, optimality_tol=1e-6, enable_polishing=True)])
+def test_packs(kw):
+    lps = [G.random_lp(m, n, lo, hi, 60 + m)[0] for m, n, lo, hi in
+           ((1, 1, 1, 1), (3, 7, 1, 2), (31, 33, 2, 9), (257, 640, 4, 12), (256, 256, 4, 30), (700, 1750, 4, 12),
+            (2100, 5000, 4, 12))] + [_holes(64, 50, 2)]
+    rng = np.random.default_rng(0)
+    warm = [None] * (len(lps) - 1) + [(rng.uniform(0, 1, 50), rng.standard_normal(64))]
+    a = batch_solve(lps, PdlpOptions(**{**LOOSE, **kw}), warm=warm)
+    b = batch_solve(lps, PdlpOptions(batch_persistent=True, **{**LOOSE, **kw}), warm=warm)
+    for (r, x, y), (q, u, v) in zip(a, b):
+        for f in FIELDS:
+            assert getattr(r, f) == getattr(q, f), f
+        np.testing.assert_array_equal(x, u)
+        np.testing.assert_array_equal(y, v)
+
+
+def test_packs_from_many_threads():
+    lps = [G.random_lp(m, int(2.5 * m), 4, 12, 70 + m)[0] for m in (300, 900, 1500, 2500, 4000)]
+    alone = batch_solve(lps, PdlpOptions(**LOOSE))
+    out = [None] * 6
+    ts = [threading.Thread(target=lambda k=k: out.__setitem__(k, batch_solve(lps, PdlpOptions(**LOOSE))))
+          for k in range(len(out))]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    for res in out:
+        for (r, x, y), (q, u, v) in zip(alone, res):
+            assert (r.iterations, r.objective) == (q.iterations, q.objective)
+            np.testing.assert_array_equal(x, u)
+            np.testing.assert_array_equal(y, v)
