@@ -29,9 +29,12 @@
 constexpr int kFam = 32;  // lanes (LPs) per family pack
 // Consecutive columns / base rows one warp of a step kernel walks as one
 // contiguous entry range (their CSR entries are adjacent), so a warp keeps
-// several rows' loads and gathers in flight instead of one short row's.
+// several rows' loads and gathers in flight instead of one short row's; one at a
+// time where a base has too few of them to give every SM kFamWarps warps (the
+// serving base of 20,000 x 50,000 keeps several, 1,000 x 2,500 takes one).
 constexpr int kFamColsPerWarp = 4;
 constexpr int kFamRowsPerWarp = 2;
+constexpr int kFamWarps = 32;
 constexpr unsigned kFull = 0xffffffffu;
 
 // Per-lane step parameters of the running cycle, structure of arrays so that a
@@ -59,6 +62,7 @@ struct FamArgs {
     const int* k_lane;    // LP of each appended row
     const int* k_first;   // [33] first appended row of each lane
     const int* kt_ptr;    // appended entries by column: row, LP, value
+    const int* kt_lptr;   // [n * 32 + 1] the same entries by column and lane
     const int* kt_row;
     const int* kt_lane;
     const double* kt_val;
@@ -80,7 +84,9 @@ struct FamArgs {
     double *pi_x, *pi_y, *pi_xn, *pi_part;
     int n, mb, K, L;
     int gb, gk;           // power blocks over base rows, appended rows (one row per warp)
-    int gp, gd;           // step blocks: columns, base rows (kFamColsPerWarp / kFamRowsPerWarp per warp)
+    int gp, gd;           // step blocks: columns, base rows (cpw / rpw per warp)
+    int cpw, rpw;
+    int listed;           // appended entries are walked by lane (famCutColumns)
     int nbr, nbk, nbc;    // check blocks: base rows, appended rows (one per lane, or none), columns
     int max_iter, polish_max_iter, N, sv_max_iter;
     double sv_tol;
@@ -215,6 +221,67 @@ __device__ __forceinline__ double famCutDot(const FamArgs& a, int q, int l, Get 
     return s;
 }
 
+// Lane l's appended entries of the R columns from j0 on (nr of them real): add(r,
+// value, row slot) in row order for each column.  Where the columns hold many
+// (kFamListed), every lane walks its own list, two entries of every column
+// loaded together; where they hold few, the warp walks the column's list and
+// every lane picks its own, which spares 256 bytes of list bounds per column.
+// Measured on B200 (us per iteration of the pack, one walk / own lists): 16 node
+// LPs of a 1,000 x 2,500 base (17 entries per column) 45.7 / 15.7, 32 of 2,000 x
+// 5,000 (17) 44.4 / 23.0, 32 of 20,000 x 50,000 (1.8) 132 / 171.
+constexpr int kFamListed = 4;  // mean appended entries per column
+template <int R, bool LISTED, class Add>
+__device__ __forceinline__ void famCutColumns(const FamArgs& a, int j0, int nr, int l, bool on, Add add) {
+    if constexpr (!LISTED) {
+        int bnd[R + 1], p;
+        famBounds<R>(a.kt_ptr, j0, a.n, l, bnd, p);
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            for (int k = bnd[r]; k < bnd[r + 1]; ++k)
+                if (on && a.kt_lane[k] == l) add(r, a.kt_val[k], fCut(a, a.kt_row[k]));
+        return;
+    }
+    int k[R], e[R];
+    bool more = false;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const bool in = on && r < nr;
+        const size_t at = static_cast<size_t>(j0 + r) * kFam + static_cast<size_t>(l);
+        k[r] = in ? __ldg(a.kt_lptr + at) : 0;
+        e[r] = in ? __ldg(a.kt_lptr + at + 1) : 0;
+        more |= k[r] < e[r];
+    }
+    while (more) {
+        int q[R][2];
+        double v[R][2];
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const bool in = k[r] + u < e[r];
+                q[r][u] = in ? __ldg(a.kt_row + k[r] + u) : -1;
+                v[r][u] = in ? __ldg(a.kt_val + k[r] + u) : 0.0;
+            }
+        more = false;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+#pragma unroll
+            for (int u = 0; u < 2; ++u)
+                if (q[r][u] >= 0) add(r, v[r][u], fCut(a, q[r][u]));
+            k[r] += 2;
+            more |= k[r] < e[r];
+        }
+    }
+}
+
+template <class Add>
+__device__ __forceinline__ void cutColumn(const FamArgs& a, int j, int l, bool on, Add add) {
+    if (a.listed)
+        famCutColumns<1, true>(a, j, 1, l, on, add);
+    else
+        famCutColumns<1, false>(a, j, 1, l, on, add);
+}
+
 // Dual proximal step of one row (pdlp_kernels.cu:94-157, as dualUpdate) given
 // s = (A_l x_refl)_i; returns the new current y, py the pdhg y.
 __device__ __forceinline__ double famDualStep(const RowPack<double>& q, double yc, double yi, double s, double step,
@@ -243,21 +310,20 @@ __device__ __forceinline__ double famDualStep(const RowPack<double>& q, double y
 }
 
 // ---- PDHG step -----------------------------------------------------------------
-// Primal: one warp per kFamColsPerWarp consecutive columns;
+// Primal: one warp per R consecutive columns;
 // (A_l^T y)_j = c_lj (sum_i a_ij ys_il + appended entries).  Lanes of LPs
 // still running gather at once (the live mask of the last cycle); the solver
 // state -- iteration limits inside the cycle, step, weight -- is read after
 // the sums, and the per-lane column data is prefetched into L2 meanwhile.
+template <int R, bool LISTED>
 __global__ void __launch_bounds__(kBlock, 4) famPrimal(FamArgs a, int koff) {
-    constexpr int R = kFamColsPerWarp;
     const int j0 = (static_cast<int>(blockIdx.x) * kWarps + static_cast<int>(threadIdx.x >> 5)) * R;
     const int l = threadIdx.x & 31;
     if (j0 >= a.n) return;
     const bool live = (*a.live >> l) & 1u;
     if (__ballot_sync(kFull, live) == 0) return;
-    int bnd[R + 1], kbd[R + 1], pl, pk;
+    int bnd[R + 1], pl;
     const int nr = famBounds<R>(a.at_ptr, j0, a.n, l, bnd, pl);
-    famBounds<R>(a.kt_ptr, j0, a.n, l, kbd, pk);
     if (live)
         for (int r = 0; r < nr; ++r) {
             const size_t q = fIdx(j0 + r, l);
@@ -269,10 +335,7 @@ __global__ void __launch_bounds__(kBlock, 4) famPrimal(FamArgs a, int koff) {
     const double* ys = a.ys;
     double s[R];
     famDotRows<R>(a.at_idx, a.at_val, bnd, pl, l, live, [&](int i) { return __ldg(ys + (static_cast<size_t>(i) + l)); }, s);
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-        for (int k = kbd[r]; k < kbd[r + 1]; ++k)
-            if (live && a.kt_lane[k] == l) s[r] += a.kt_val[k] * ys[fCut(a, a.kt_row[k])];
+    famCutColumns<R, LISTED>(a, j0, nr, l, live, [&](int r, double v, size_t q) { s[r] += v * ys[q]; });
     const int allow = a.lanes->allow[l];
     if (!live || koff > allow) return;
     const bool last = koff == allow;
@@ -296,14 +359,14 @@ __global__ void __launch_bounds__(kBlock, 4) famPrimal(FamArgs a, int koff) {
     }
 }
 
-// Dual: blocks [0, gd) one warp per kFamRowsPerWarp base rows, then one warp
+// Dual: blocks [0, gd) one warp per R base rows, then one warp
 // per appended row.
+template <int R>
 __global__ void __launch_bounds__(kBlock, 4) famDual(FamArgs a, int koff) {
     const int w = static_cast<int>(threadIdx.x >> 5);
     const int l = threadIdx.x & 31;
     const double* xs = a.xs;
     if (static_cast<int>(blockIdx.x) < a.gd) {
-        constexpr int R = kFamRowsPerWarp;
         const int i0 = (static_cast<int>(blockIdx.x) * kWarps + w) * R;
         if (i0 >= a.mb) return;
         const bool live = (*a.live >> l) & 1u;
@@ -449,12 +512,10 @@ __global__ void __launch_bounds__(kBlock) famCheckCols(FamArgs a) {
             const size_t q = static_cast<size_t>(i) + l;
             return rs[q] * (yh[q] - yi[q]);
         });
-        for (int k = a.kt_ptr[j]; k < a.kt_ptr[j + 1]; ++k) {
-            if (!on || a.kt_lane[k] != l) continue;
-            const size_t q = fCut(a, a.kt_row[k]);
-            aty += a.kt_val[k] * (rs[q] * yh[q]);
-            atdy += a.kt_val[k] * (rs[q] * (yh[q] - yi[q]));
-        }
+        cutColumn(a, j, l, on, [&](int, double v, size_t q) {
+            aty += v * (rs[q] * yh[q]);
+            atdy += v * (rs[q] * (yh[q] - yi[q]));
+        });
         if (on) {
             const size_t c = fIdx(j, l);
             const ColPack<double> p = a.cp[c];
@@ -602,11 +663,7 @@ __global__ void __launch_bounds__(kBlock) famPowerAt(FamArgs a) {
             const size_t q = static_cast<size_t>(i) + l;
             return rs[q] * py[q];
         });
-        for (int k = a.kt_ptr[j]; k < a.kt_ptr[j + 1]; ++k)
-            if (on && a.kt_lane[k] == l) {
-                const size_t q = fCut(a, a.kt_row[k]);
-                s += a.kt_val[k] * (rs[q] * py[q]);
-            }
+        cutColumn(a, j, l, on, [&](int, double v, size_t q) { s += v * (rs[q] * py[q]); });
         if (on) {
             const size_t c = fIdx(j, l);
             const double xn = a.cs[c] * s;
@@ -698,7 +755,7 @@ struct FamPack {
     int64_t Zb = 0, Zk = 0, Zkcap = 0;
     std::vector<int> qfirst;    // first appended row of each lane (kFam + 1 entries)
     size_t o_aptr, o_aidx, o_aval, o_atptr, o_atidx, o_atval, o_kptr, o_kidx, o_kval, o_klane, o_kfirst, o_live, o_lanes;
-    size_t o_ktptr, o_ktrow, o_ktlane, o_ktval, o_cp, o_cs, o_rp, o_rs, o_st, o_dc, o_ps, o_pix;
+    size_t o_ktptr, o_ktlptr, o_ktrow, o_ktlane, o_ktval, o_cp, o_cs, o_rp, o_rs, o_st, o_dc, o_ps, o_pix;
     size_t image_end;
     size_t o_xc, o_xi, o_xh, o_xs, o_yc, o_yi, o_yh, o_ys;
     size_t iter_end;
@@ -745,6 +802,7 @@ struct FamPack {
         o_live = take(4);
         o_lanes = take(sizeof(FamLane));
         o_ktptr = take(4 * (static_cast<size_t>(n) + 1));
+        o_ktlptr = take(4 * (colsAll() + 1));
         o_ktrow = take(4 * static_cast<size_t>(Zkcap));
         o_ktlane = take(4 * static_cast<size_t>(Zkcap));
         o_ktval = take(8 * static_cast<size_t>(Zkcap));
@@ -782,7 +840,7 @@ struct FamPack {
 size_t familyPackBytes(int64_t n, int64_t mb, int64_t zb, int64_t K, int64_t zk, int nbc, int nbrk) {
     const size_t C = static_cast<size_t>(n) * kFam, R = static_cast<size_t>(mb) * kFam + static_cast<size_t>(K);
     size_t b = 4 * static_cast<size_t>(mb + n + 2) + 24 * static_cast<size_t>(zb);
-    b += 4 * static_cast<size_t>(K + n + 2) + 28 * static_cast<size_t>(zk) + 4 * static_cast<size_t>(K);
+    b += 4 * (static_cast<size_t>(K) + C + 2) + 28 * static_cast<size_t>(zk) + 4 * static_cast<size_t>(K);
     b += C * (32 + 8 + 8 * 6) + R * (32 + 8 + 8 * 5);
     b += 8 * kFam * (2 * static_cast<size_t>(nbc) + kRowSlots * static_cast<size_t>(nbrk) + kColSlots * static_cast<size_t>(nbc));
     return b + 64 * 1024;
@@ -834,9 +892,9 @@ void famLaneData(const Item& it, int n, FamLaneData& q) {
 
 // The appended rows of the lanes in use (lane order; a lane without a member
 // contributes none): row pointers, entries, lanes, per-lane first row, and the
-// same entries by column (row order inside a column).
+// same entries by column and lane (row order inside both).
 struct FamCuts {
-    std::vector<int32_t> kp, ki, kl, kf, ktp, ktr, ktl;
+    std::vector<int32_t> kp, ki, kl, kf, ktp, ktlp, ktr, ktl;
     std::vector<double> kv, ktv;
     int K = 0;
     int64_t Zk = 0;
@@ -849,7 +907,7 @@ void famBuildCuts(const FamPack& fp, const std::vector<char>& in_use, FamCuts& c
     c.kv.clear();
     c.kl.clear();
     c.kf.assign(kFam + 1, 0);
-    std::vector<int32_t> colcnt(static_cast<size_t>(n) + 1, 0);
+    std::vector<int32_t> colcnt(static_cast<size_t>(n) * kFam + 1, 0);
     int q = 0;
     for (int l = 0; l < kFam; ++l) {
         c.kf[l] = q;
@@ -861,7 +919,7 @@ void famBuildCuts(const FamPack& fp, const std::vector<char>& in_use, FamCuts& c
             for (int32_t k = a.ptr[i]; k < a.ptr[i + 1]; ++k) {
                 c.ki.push_back(a.idx[k]);
                 c.kv.push_back(a.val[k]);
-                ++colcnt[a.idx[k] + 1];
+                ++colcnt[static_cast<size_t>(a.idx[k]) * kFam + l + 1];
             }
         }
     }
@@ -869,14 +927,16 @@ void famBuildCuts(const FamPack& fp, const std::vector<char>& in_use, FamCuts& c
     c.K = q;
     c.Zk = static_cast<int64_t>(c.ki.size());
     c.kp.push_back(static_cast<int32_t>(c.Zk));
-    for (int32_t j = 0; j < n; ++j) colcnt[j + 1] += colcnt[j];
-    c.ktp = colcnt;
+    for (size_t j = 1; j < colcnt.size(); ++j) colcnt[j] += colcnt[j - 1];
+    c.ktlp = colcnt;
+    c.ktp.resize(static_cast<size_t>(n) + 1);
+    for (int32_t j = 0; j <= n; ++j) c.ktp[j] = colcnt[static_cast<size_t>(j) * kFam];
     c.ktr.resize(static_cast<size_t>(c.Zk));
     c.ktl.resize(static_cast<size_t>(c.Zk));
     c.ktv.resize(static_cast<size_t>(c.Zk));
     for (int qq = 0; qq < c.K; ++qq)
         for (int32_t k = c.kp[qq]; k < c.kp[qq + 1]; ++k) {
-            const int32_t at = colcnt[c.ki[k]]++;
+            const int32_t at = colcnt[static_cast<size_t>(c.ki[k]) * kFam + c.kl[qq]]++;
             c.ktr[at] = qq;
             c.ktl[at] = c.kl[qq];
             c.ktv[at] = c.kv[k];
@@ -917,8 +977,9 @@ int32_t solveFamilyPack(FamPack& fp, const pdlpx_options& o, std::chrono::steady
     fp.Zkcap = std::max<int64_t>(2 * cuts.Zk, static_cast<int64_t>(kFam) * 64 * 256);
     fp.Zb = fb.ptr[mb];
     const int gb = famBlocks(mb);
-    const int gp = famBlocks((static_cast<int64_t>(n) + kFamColsPerWarp - 1) / kFamColsPerWarp);
-    const int gd = famBlocks((static_cast<int64_t>(mb) + kFamRowsPerWarp - 1) / kFamRowsPerWarp);
+    const int cpw = n <= kFamWarps * sms ? 1 : kFamColsPerWarp, rpw = mb <= kFamWarps * sms ? 1 : kFamRowsPerWarp;
+    const int gp = famBlocks((static_cast<int64_t>(n) + cpw - 1) / cpw);
+    const int gd = famBlocks((static_cast<int64_t>(mb) + rpw - 1) / rpw);
     const int cap = 4 * sms;
     const int nbr = std::min(gb, cap), nbc = std::min(famBlocks(n), cap);
     fp.layout(nbr, nbc);
@@ -953,6 +1014,7 @@ int32_t solveFamilyPack(FamPack& fp, const pdlpx_options& o, std::chrono::steady
     std::memcpy(I(fp.o_kfirst), cuts.kf.data(), 4 * cuts.kf.size());
     *reinterpret_cast<uint32_t*>(H + fp.o_live) = L >= kFam ? ~0u : ((1u << L) - 1u);
     std::memcpy(I(fp.o_ktptr), cuts.ktp.data(), 4 * cuts.ktp.size());
+    std::memcpy(I(fp.o_ktlptr), cuts.ktlp.data(), 4 * cuts.ktlp.size());
     std::memcpy(I(fp.o_ktrow), cuts.ktr.data(), 4 * cuts.ktr.size());
     std::memcpy(I(fp.o_ktlane), cuts.ktl.data(), 4 * cuts.ktl.size());
     std::memcpy(D(fp.o_ktval), cuts.ktv.data(), 8 * cuts.ktv.size());
@@ -1059,6 +1121,7 @@ int32_t solveFamilyPack(FamPack& fp, const pdlpx_options& o, std::chrono::steady
         a.live = reinterpret_cast<const unsigned*>(d + fp.o_live);
         a.lanes = reinterpret_cast<FamLane*>(d + fp.o_lanes);
         a.kt_ptr = Pi(fp.o_ktptr);
+        a.kt_lptr = Pi(fp.o_ktlptr);
         a.kt_row = Pi(fp.o_ktrow);
         a.kt_lane = Pi(fp.o_ktlane);
         a.kt_val = Pd(fp.o_ktval);
@@ -1090,6 +1153,8 @@ int32_t solveFamilyPack(FamPack& fp, const pdlpx_options& o, std::chrono::steady
         a.gb = gb;
         a.gp = gp;
         a.gd = gd;
+        a.cpw = cpw;
+        a.rpw = rpw;
         a.nbr = nbr;
         a.nbc = nbc;
         a.max_iter = o.max_iter;
@@ -1103,6 +1168,7 @@ int32_t solveFamilyPack(FamPack& fp, const pdlpx_options& o, std::chrono::steady
         a.K = fp.K;
         a.L = L;
         a.gk = fp.K > 0 ? famBlocks(fp.K) : 0;
+        a.listed = fp.Zk >= static_cast<int64_t>(kFamListed) * n;
         a.nbk = L;  // one check block per lane for its appended rows (identity partials when it has none)
     };
     setShape(fp.args);
@@ -1152,8 +1218,14 @@ int32_t solveFamilyPack(FamPack& fp, const pdlpx_options& o, std::chrono::steady
             }
         } else {
             for (int k = 1; k <= o.termination_eval_frequency; ++k) {
-                famPrimal<<<args.gp, kBlock, 0, s>>>(args, k);
-                famDual<<<args.gd + args.gk, kBlock, 0, s>>>(args, k);
+                auto primal = args.cpw == 1 ? (args.listed ? famPrimal<1, true> : famPrimal<1, false>)
+                                            : (args.listed ? famPrimal<kFamColsPerWarp, true>
+                                                           : famPrimal<kFamColsPerWarp, false>);
+                primal<<<args.gp, kBlock, 0, s>>>(args, k);
+                if (args.rpw == 1)
+                    famDual<1><<<args.gd + args.gk, kBlock, 0, s>>>(args, k);
+                else
+                    famDual<kFamRowsPerWarp><<<args.gd + args.gk, kBlock, 0, s>>>(args, k);
                 count += 2;
             }
             famCheckRows<<<args.nbr + args.nbk, kBlock, 0, s>>>(args);
@@ -1280,6 +1352,7 @@ int32_t solveFamilyPack(FamPack& fp, const pdlpx_options& o, std::chrono::steady
         PDLPX_BCK(up(d + fp.o_klane, c.kl.data(), 4 * c.kl.size()));
         PDLPX_BCK(up(d + fp.o_kfirst, c.kf.data(), 4 * c.kf.size()));
         PDLPX_BCK(up(d + fp.o_ktptr, c.ktp.data(), 4 * c.ktp.size()));
+        PDLPX_BCK(up(d + fp.o_ktlptr, c.ktlp.data(), 4 * c.ktlp.size()));
         PDLPX_BCK(up(d + fp.o_ktrow, c.ktr.data(), 4 * c.ktr.size()));
         PDLPX_BCK(up(d + fp.o_ktlane, c.ktl.data(), 4 * c.ktl.size()));
         PDLPX_BCK(up(d + fp.o_ktval, c.ktv.data(), 8 * c.ktv.size()));
