@@ -16,6 +16,7 @@
 #include <cstdio>
 #include <cstring>
 #include <functional>
+#include <future>
 #include <thread>
 #include <limits>
 #include <random>
@@ -566,7 +567,7 @@ struct DeviceLp {
     double *yc64 = nullptr, *yi64 = nullptr, *yh64 = nullptr;
     float* yg32 = nullptr;  // FP32 copy of yc, gathered by the mixed-mode primal step
     double *prev_ax = nullptr, *prev_xh = nullptr;
-    double *pi_x = nullptr, *pi_y = nullptr, *pi_xn = nullptr, *pi_part = nullptr, *pi_rpart = nullptr;
+    double *pi_x0 = nullptr, *pi_x = nullptr, *pi_y = nullptr, *pi_xn = nullptr, *pi_part = nullptr, *pi_rpart = nullptr;
     double *part_rows = nullptr, *part_cols = nullptr;
     // Anderson acceleration at restarts (anderson.cuh); aa_w = 0 when off.
     int aa_w = 0, aa_nb = 1;
@@ -1125,21 +1126,13 @@ void packRows(const ScaledLp& sc, std::vector<RowPack<T>>& out) {
                             static_cast<T>(sc.row_type[i])};
 }
 
-// Vectors between the original numbering and the device numbering
-// (pos: original -> device; empty = identity).
+// A vector into the device numbering (pos: original -> device; empty = identity).
 void toDevice(std::vector<double>& v, const std::vector<int32_t>& pos) {
     if (pos.empty()) return;
     std::vector<double> w(v.size());
     for (size_t k = 0; k < v.size(); ++k) w[pos[k]] = v[k];
     v.swap(w);
 }
-void fromDevice(std::vector<double>& v, const std::vector<int32_t>& pos) {
-    if (pos.empty()) return;
-    std::vector<double> w(v.size());
-    for (size_t k = 0; k < v.size(); ++k) w[k] = v[pos[k]];
-    v.swap(w);
-}
-
 bool timeUp(std::chrono::steady_clock::time_point t0, double lim) {
     if (lim < 0.0) return false;
     return std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count() >= lim;
@@ -1431,6 +1424,21 @@ static bool wantMixed(const pdlpx_options& o, int64_t m, int64_t n, int64_t nnz)
     return 24 * nnz + 64 * n + 56 * m >= kMixedMinBytes;
 }
 
+// Start vector of the power iteration: mt19937(42) normals, normalised
+// (pdlp.cpp:1990-2001), in the original numbering.
+static std::vector<double> startVector(int32_t n) {
+    std::mt19937 rng(42);
+    std::normal_distribution<double> dist(0.0, 1.0);
+    std::vector<double> x(static_cast<size_t>(n));
+    for (auto& v : x) v = dist(rng);
+    double xn = 0.0;
+    for (double v : x) xn += v * v;
+    xn = std::sqrt(xn);
+    if (xn < 1e-15) xn = 1.0;
+    for (auto& v : x) v /= xn;
+    return x;
+}
+
 // Build (or rebuild) the device image of the scaled LP.
 static int32_t buildDevice(std::unique_ptr<DeviceLp>& dp, const ScaledLp& sc_in, const pdlpx_options& o,
                            std::string& err) {
@@ -1440,6 +1448,11 @@ static int32_t buildDevice(std::unique_ptr<DeviceLp>& dp, const ScaledLp& sc_in,
         err = "no CUDA device visible";
         return PDLPX_E_NO_DEVICE;
     }
+    // The start vector depends on the column count alone: it is part of the image
+    // (every solve generated it anew before, 14 ms for 1M columns), and for a
+    // large LP its own thread makes it while the rest is built.
+    std::future<std::vector<double>> start = std::async(
+        sc_in.a.cols >= (1 << 16) ? std::launch::async : std::launch::deferred, startVector, sc_in.a.cols);
     const int dev = (o.device >= 0 && o.device < count) ? o.device : 0;
     PDLPX_CK(cudaSetDevice(dev));
     dp.reset(new DeviceLp());
@@ -1558,7 +1571,7 @@ static int32_t buildDevice(std::unique_ptr<DeviceLp>& dp, const ScaledLp& sc_in,
     for (auto& v : o_y64) v = take(8 * m);
     const bool adaptive = o.adaptive_step != 0;
     const size_t o_prev_ax = adaptive ? take(8 * m) : 0, o_prev_xh = adaptive ? take(8 * n) : 0;
-    const size_t o_pi_x = take(8 * n), o_pi_y = take(8 * m), o_pi_xn = take(8 * n),
+    const size_t o_pi_x0 = take(8 * n), o_pi_x = take(8 * n), o_pi_y = take(8 * m), o_pi_xn = take(8 * n),
                  o_pi_part = take(8 * 4 * d.nb_pi);  // dot partials, residual partials by parity
     // cells of the linked cycle
     const bool link = linkable(d, o);
@@ -1639,6 +1652,7 @@ static int32_t buildDevice(std::unique_ptr<DeviceLp>& dp, const ScaledLp& sc_in,
         d.prev_ax = reinterpret_cast<double*>(b + o_prev_ax);
         d.prev_xh = reinterpret_cast<double*>(b + o_prev_xh);
     }
+    d.pi_x0 = reinterpret_cast<double*>(b + o_pi_x0);
     d.pi_x = reinterpret_cast<double*>(b + o_pi_x);
     d.pi_y = reinterpret_cast<double*>(b + o_pi_y);
     d.pi_xn = reinterpret_cast<double*>(b + o_pi_xn);
@@ -1756,6 +1770,9 @@ static int32_t buildDevice(std::unique_ptr<DeviceLp>& dp, const ScaledLp& sc_in,
         PDLPX_CK(up(d.ru64, sc.ru.data(), 8 * m));
         PDLPX_CK(up(d.rs64, sc.row_scale.data(), 8 * m));
         PDLPX_CK(up(d.sig64, sc.sigma.data(), 8 * m));
+        std::vector<double> x0 = start.get();
+        toDevice(x0, d.cpos);
+        PDLPX_CK(up(d.pi_x0, x0.data(), 8 * n));
         PDLPX_CK(cudaStreamSynchronize(s));
     }
     if (o.verbose) {
@@ -2155,20 +2172,10 @@ int32_t Engine::solveDevice(pdlpx_result* out) {
     } ev_guard{ev0, ev1};
     PDLPX_CK(cudaEventRecord(ev0, s));
 
-    // ---- power iteration (start vector: mt19937(42) normals, pdlp.cpp:1990-2001)
+    // ---- power iteration from the image's start vector
     double step = 1.0;
     {
-        std::mt19937 rng(42);
-        std::normal_distribution<double> dist(0.0, 1.0);
-        std::vector<double> x0(static_cast<size_t>(n));
-        for (auto& v : x0) v = dist(rng);
-        double xn = 0.0;
-        for (double v : x0) xn += v * v;
-        xn = std::sqrt(xn);
-        if (xn < 1e-15) xn = 1.0;
-        for (auto& v : x0) v /= xn;
-        toDevice(x0, d.cpos);
-        PDLPX_CK(cudaMemcpyAsync(d.pi_x, x0.data(), 8 * static_cast<size_t>(n), cudaMemcpyHostToDevice, s));
+        PDLPX_CK(cudaMemcpyAsync(d.pi_x, d.pi_x0, 8 * static_cast<size_t>(n), cudaMemcpyDeviceToDevice, s));
         PowerState ps0{1.0, 0.0, 0.0, 0, opt_.sv_max_iter <= 0 ? 1 : 0};
         *d.h_ps = ps0;
         PDLPX_CK(cudaMemcpyAsync(d.ps, d.h_ps, sizeof(PowerState), cudaMemcpyHostToDevice, s));
@@ -2283,12 +2290,19 @@ int32_t Engine::solveDevice(pdlpx_result* out) {
         toDevice(wx, d.cpos);
         toDevice(wy, d.rpos);
     }
-    if (d.mixed) {
-        std::vector<float> fx(n, 0.0f), fy(m, 0.0f);
-        if (warm) {
-            for (int32_t j = 0; j < n; ++j) fx[j] = static_cast<float>(wx[j]);
-            for (int32_t i = 0; i < m; ++i) fy[i] = static_cast<float>(wy[i]);
+    if (!warm) {
+        const size_t bx = static_cast<size_t>(n), by = static_cast<size_t>(m);
+        if (d.mixed) {
+            for (float* p : {d.xi32, d.xh32, d.xr32}) PDLPX_CK(cudaMemsetAsync(p, 0, 4 * bx, s));
+            for (float* p : {d.yi32, d.yh32, d.yg32}) PDLPX_CK(cudaMemsetAsync(p, 0, 4 * by, s));
+            PDLPX_CK(cudaMemsetAsync(d.xc64, 0, 8 * bx, s));
+            PDLPX_CK(cudaMemsetAsync(d.yc64, 0, 8 * by, s));
+        } else {
+            for (double* p : {d.xc64, d.xi64, d.xh64, d.xr64}) PDLPX_CK(cudaMemsetAsync(p, 0, 8 * bx, s));
+            for (double* p : {d.yc64, d.yi64, d.yh64}) PDLPX_CK(cudaMemsetAsync(p, 0, 8 * by, s));
         }
+    } else if (d.mixed) {
+        std::vector<float> fx(wx.begin(), wx.end()), fy(wy.begin(), wy.end());
         for (float* p : {d.xi32, d.xh32, d.xr32})
             PDLPX_CK(cudaMemcpyAsync(p, fx.data(), 4 * static_cast<size_t>(n), cudaMemcpyHostToDevice, s));
         for (float* p : {d.yi32, d.yh32})
@@ -2300,10 +2314,6 @@ int32_t Engine::solveDevice(pdlpx_result* out) {
         PDLPX_CK(cudaMemcpyAsync(d.yg32, fy.data(), 4 * static_cast<size_t>(m), cudaMemcpyHostToDevice, s));
         PDLPX_CK(cudaStreamSynchronize(s));
     } else {
-        if (!warm) {
-            wx.assign(n, 0.0);
-            wy.assign(m, 0.0);
-        }
         for (double* p : {d.xc64, d.xi64, d.xh64, d.xr64})
             PDLPX_CK(cudaMemcpyAsync(p, wx.data(), 8 * static_cast<size_t>(n), cudaMemcpyHostToDevice, s));
         for (double* p : {d.yc64, d.yi64, d.yh64})
@@ -2421,48 +2431,62 @@ int32_t Engine::solveDevice(pdlpx_result* out) {
     }
 
     // ---- results (pdlp.cpp:2678-2712)
-    const int fprec = fin.prec;
-    std::vector<double> xh(n), yh(m);
-    if (status == PDLPX_STATUS_OPTIMAL || status == PDLPX_STATUS_INFEASIBLE || status == PDLPX_STATUS_UNBOUNDED) {
-        if (fprec == 0) {
-            std::vector<float> fx(n), fy(m);
+    // x_hat, y_hat as the device holds them; the loops below read them in the
+    // original numbering, on host threads for large LPs
+    const bool solved =
+        status == PDLPX_STATUS_OPTIMAL || status == PDLPX_STATUS_INFEASIBLE || status == PDLPX_STATUS_UNBOUNDED;
+    const bool f32 = fin.prec == 0;
+    std::vector<float> fx, fy;
+    std::vector<double> dx, dy;
+    if (solved) {
+        if (f32) {
+            fx.resize(n);
+            fy.resize(m);
             PDLPX_CK(cudaMemcpyAsync(fx.data(), d.xh32, 4 * static_cast<size_t>(n), cudaMemcpyDeviceToHost, s));
             PDLPX_CK(cudaMemcpyAsync(fy.data(), d.yh32, 4 * static_cast<size_t>(m), cudaMemcpyDeviceToHost, s));
-            PDLPX_CK(cudaStreamSynchronize(s));
-            for (int32_t j = 0; j < n; ++j) xh[j] = fx[j];
-            for (int32_t i = 0; i < m; ++i) yh[i] = fy[i];
         } else {
-            PDLPX_CK(cudaMemcpyAsync(xh.data(), d.xh64, 8 * static_cast<size_t>(n), cudaMemcpyDeviceToHost, s));
-            PDLPX_CK(cudaMemcpyAsync(yh.data(), d.yh64, 8 * static_cast<size_t>(m), cudaMemcpyDeviceToHost, s));
-            PDLPX_CK(cudaStreamSynchronize(s));
+            dx.resize(n);
+            dy.resize(m);
+            PDLPX_CK(cudaMemcpyAsync(dx.data(), d.xh64, 8 * static_cast<size_t>(n), cudaMemcpyDeviceToHost, s));
+            PDLPX_CK(cudaMemcpyAsync(dy.data(), d.yh64, 8 * static_cast<size_t>(m), cudaMemcpyDeviceToHost, s));
         }
-        fromDevice(xh, d.cpos);
-        fromDevice(yh, d.rpos);
+        PDLPX_CK(cudaStreamSynchronize(s));
     }
+    auto xh = [&](int64_t j) -> double {
+        const size_t k = static_cast<size_t>(d.cpos.empty() ? j : d.cpos[static_cast<size_t>(j)]);
+        return f32 ? fx[k] : dx[k];
+    };
+    auto yh = [&](int64_t i) -> double {
+        const size_t k = static_cast<size_t>(d.rpos.empty() ? i : d.rpos[static_cast<size_t>(i)]);
+        return f32 ? fy[k] : dy[k];
+    };
+    const double ic = 1.0 / sc_.con_scale, io = 1.0 / sc_.obj_scale;
+    auto unscaleY = [&]() {
+        y_orig_.resize(m);
+        hostBlocks(static_cast<size_t>(m), m, [&](int64_t b, int64_t e) {
+            for (int64_t i = b; i < e; ++i) y_orig_[i] = sc_.obj_sign * yh(i) * sc_.row_scale[i] * io;
+        });
+    };
     objective_ = 0.0;
     if (status == PDLPX_STATUS_OPTIMAL) {
         x_orig_.resize(n);
-        const double ic = 1.0 / sc_.con_scale;
-        for (int32_t j = 0; j < n; ++j) {
-            double xj = xh[j] * sc_.col_scale[j] * ic;
-            if (std::isfinite(lp_.cl[j])) xj = std::max(xj, lp_.cl[j]);
-            if (std::isfinite(lp_.cu[j])) xj = std::min(xj, lp_.cu[j]);
-            x_orig_[j] = xj;
-        }
-        y_orig_.resize(m);
-        const double io = 1.0 / sc_.obj_scale;
-        for (int32_t i = 0; i < m; ++i) y_orig_[i] = sc_.obj_sign * yh[i] * sc_.row_scale[i] * io;
+        hostBlocks(static_cast<size_t>(n), n, [&](int64_t b, int64_t e) {
+            for (int64_t j = b; j < e; ++j) {
+                double xj = xh(j) * sc_.col_scale[j] * ic;
+                if (std::isfinite(lp_.cl[j])) xj = std::max(xj, lp_.cl[j]);
+                if (std::isfinite(lp_.cu[j])) xj = std::min(xj, lp_.cu[j]);
+                x_orig_[j] = xj;
+            }
+        });
+        unscaleY();
         double ov = lp_.offset;
         for (int32_t j = 0; j < n; ++j) ov += lp_.obj[j] * x_orig_[j];
         objective_ = ov;
     } else if (status == PDLPX_STATUS_INFEASIBLE) {
-        y_orig_.resize(m);
-        const double io = 1.0 / sc_.obj_scale;
-        for (int32_t i = 0; i < m; ++i) y_orig_[i] = sc_.obj_sign * yh[i] * sc_.row_scale[i] * io;
+        unscaleY();
     } else if (status == PDLPX_STATUS_UNBOUNDED) {
         x_orig_.resize(n);
-        const double ic = 1.0 / sc_.con_scale;
-        for (int32_t j = 0; j < n; ++j) x_orig_[j] = xh[j] * sc_.col_scale[j] * ic;
+        for (int32_t j = 0; j < n; ++j) x_orig_[j] = xh(j) * sc_.col_scale[j] * ic;
     }
     status_ = status;
     iterations_ = fin.total;
