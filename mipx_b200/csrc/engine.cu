@@ -404,6 +404,28 @@ __global__ void __launch_bounds__(linkThreads(CSR), 1) linkedSteps(LinkArgs<T> a
     linkedCycle<LP, LD, CSR, T>(a);
 }
 
+// The long columns as CSR rows of G lanes (blocks [0, lblocks)) and the short ones
+// in sliced ELL, in one launch: one after the other, each leaves SMs idle (a
+// mid-size LP's launches hold a few blocks per SM) and pays its own ramp.  The
+// gathers' sectors from L2 bound it then, 32 bytes each at 6-7 TB/s.  Same
+// per-thread work as the two launches.  Measured on B200 (power-law LPs, us per
+// iteration, apart -> in one): 25k x 100k 31.0 -> 21.9, 60k x 200k 38.1 -> 25.2,
+// 100k x 400k 54.2 -> 49.1, 200k x 700k 98.1 -> 73.9; 25k x 100k in FP64
+// 29.5 -> 21.7.
+template <int G, int UL, int U, class T>
+__global__ void __launch_bounds__(kBlock, sellMinBlocks<T, true>())
+    primalLongShort(IterArgs<T> p, const int2* __restrict__ hdr, const int* __restrict__ idx,
+                    const T* __restrict__ val, int koff, int begin, int end, int lblocks) {
+    const int b = static_cast<int>(blockIdx.x);
+    if (b < lblocks) {
+        primalRows<G, 1, UL, T, true>(p, b * (kBlock / G) + static_cast<int>(threadIdx.x) / G, begin, koff);
+        return;
+    }
+    const int r = (b - lblocks) * kBlock + static_cast<int>(threadIdx.x);
+    if (begin + r >= end) return;
+    primalSellFrom<U, T, false, false, true>(p, idx, val, begin + r, hdr[r / kSlice], koff);
+}
+
 // ---- power iteration over the sliced-ELL sides --------------------------------
 // The short rows of A (y = A x) and of A^T (x_n = A^T y, with the block
 // partials of x . x_n and x_n . x_n) in the step kernels' layout: one thread
@@ -861,6 +883,13 @@ void launchDualShort(const DeviceLp& d, const IterArgs<T>& ia, int shape, int k,
     }
 }
 
+// Whether the long columns' CSR launch and the short columns' sliced-ELL launch
+// run as one (the shapes longShape and sellShape pick).
+template <class T>
+bool primalFused(const DeviceLp& d) {
+    return (d.shapeP == kNumShapes || d.shapeP == kNumShapes + 1) && hotPrimal<T>(d) == 0 &&
+           (d.shapeLP == 9 || d.shapeLP == 11 || d.shapeLP == 13 || d.shapeLP == 15);
+}
 // Step launches of one iteration on each side: the long rows (if any), then the rest.
 template <class T>
 int launchPrimal(const DeviceLp& d, const IterArgs<T>& ia, int k, cudaStream_t s) {
@@ -884,6 +913,20 @@ int launchPrimal(const DeviceLp& d, const IterArgs<T>& ia, int k, cudaStream_t s
             }
             return n;
         }
+    }
+    if (d.nlP > 0 && d.n > d.nlP && primalFused<T>(d)) {
+        const int lb = gridForShape(d.nlP, d.shapeLP), grid = lb + sellGrid(d.n - d.nlP);
+        auto fused = [&](auto kernel) {
+            kernel<<<grid, kBlock, 0, s>>>(ia, d.sp_hdr, d.sp_idx, sellVals<T>(d, true), k, d.nlP, d.n, lb);
+        };
+        const bool u8 = d.shapeP == kNumShapes + 1;
+        switch (d.shapeLP) {
+            case 9: u8 ? fused(primalLongShort<32, 4, 8, T>) : fused(primalLongShort<32, 4, 4, T>); break;
+            case 11: u8 ? fused(primalLongShort<64, 4, 8, T>) : fused(primalLongShort<64, 4, 4, T>); break;
+            case 13: u8 ? fused(primalLongShort<128, 8, 8, T>) : fused(primalLongShort<128, 8, 4, T>); break;
+            default: u8 ? fused(primalLongShort<256, 8, 8, T>) : fused(primalLongShort<256, 8, 4, T>); break;
+        }
+        return n + 1;
     }
     if (d.nlP > 0) {
         PDLPX_SHAPE_SWITCH(d.shapeLP,

@@ -173,3 +173,17 @@ def test_packs_from_many_threads():
             assert (r.iterations, r.objective) == (q.iterations, q.objective)
             np.testing.assert_array_equal(x, u)
             np.testing.assert_array_equal(y, v)
+
+
+# long and short columns of the primal step in one launch, against the two launches
+# that a pinned sliced-ELL variant other than the table's takes (19: 16 entries per round)
+@pytest.mark.parametrize("m,kmax,kmean", [(9000, 90, 10.0), (9000, 2000, 10.0), (6000, 6000, 30.0)])
+@pytest.mark.parametrize("precision", [Precision.Mixed, Precision.FP64])
+def test_long_and_short_columns_in_one_launch(m, kmax, kmean, precision):
+    lp, _ = G.powerlaw_lp(m, 4 * m + 5, kmax=kmax, kmean=kmean, seed=m + kmax)
+    pins = dict(shape_dual=18, precision=precision, max_iter=400, termination_eval_frequency=100)
+    a, sa = _solve(lp, shape_primal=17, **pins)
+    b, sb = _solve(lp, shape_primal=19, **pins)
+    assert a.kernel_launches < b.kernel_launches, "the launches did not run as one"
+    for f in FIELDS:
+        assert getattr(a, f) == getattr(b, f), f
