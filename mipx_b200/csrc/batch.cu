@@ -102,6 +102,7 @@ struct PackArgs {
     double* pi_y;
     double* pi_xn;
     double* pi_part;      // [column tile][2]
+    double* pi_rpart;     // [2][column tile] residual partials, by the iteration's parity
     int L, nct, nrt, mixed, sv_max_iter;
     double sv_tol;
 };
@@ -575,24 +576,23 @@ __global__ void packModes(PackArgs a) {
 }
 
 // ---- power iteration on A^T A per LP (pdlp.cpp:748-795, 1985-2041) ---------------
+// A x over a tile's rows, a block per pass (one block for all passes of a tile, a
+// chain of 4-8 times three L2 latencies, took 20 us on a 64-LP pack, this 15).
 template <int G>
-__global__ void __launch_bounds__(kBlock) packPowerA(PackArgs a, int tile0) {
-    const int4 t = a.rtinfo[tile0 + blockIdx.x];
+__global__ void __launch_bounds__(kBlock) packPowerA(PackArgs a, int tile0, int passes) {
+    const int4 t = a.rtinfo[tile0 + static_cast<int>(blockIdx.x) / passes];
     if (a.ps[t.x].done) return;
-    constexpr int per = kBlock / G;
+    const int i = t.z + static_cast<int>(blockIdx.x) % passes * (kBlock / G) + static_cast<int>(threadIdx.x) / G;
     const int lane = threadIdx.x % G;
-    for (int base = t.z; base < t.w; base += per) {
-        const int i = base + threadIdx.x / G;
-        const bool valid = i < t.w;
-        double s = 0.0;
-        if (valid) {
-            const int b = a.it64.a_ptr[i], e = a.it64.a_ptr[i + 1];
-            s = a.mixed ? rowDot<G, double>(b, e, lane, a.it32.a_idx, a.it32.a_val, a.pi_x)
-                        : rowDot<G, double>(b, e, lane, a.it64.a_idx, a.it64.a_val, a.pi_x);
-        }
-        s = groupSum<G>(s);
-        if (valid && lane == 0) a.pi_y[i] = s;
+    const bool valid = i < t.w;
+    double s = 0.0;
+    if (valid) {
+        const int b = a.it64.a_ptr[i], e = a.it64.a_ptr[i + 1];
+        s = a.mixed ? rowDot<G, double>(b, e, lane, a.it32.a_idx, a.it32.a_val, a.pi_x)
+                    : rowDot<G, double>(b, e, lane, a.it64.a_idx, a.it64.a_val, a.pi_x);
     }
+    s = groupSum<G>(s);
+    if (valid && lane == 0) a.pi_y[i] = s;
 }
 
 template <int G>
@@ -623,26 +623,65 @@ __global__ void __launch_bounds__(kBlock) packPowerAt(PackArgs a, int tile0) {
     blockReduceSlots<2>(acc, ops, a.pi_part + static_cast<size_t>(tile) * 2);
 }
 
-__global__ void __launch_bounds__(32 * kCtlWarps) packPowerFinish1(PackArgs a) {
-    const int l = blockIdx.x * kCtlWarps + static_cast<int>(threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (l >= a.L || a.ps[l].done) return;
-    const int4 t = a.lpt[l];
-    const int ops[2] = {OP_SUM, OP_SUM};
-    double out[2];
-    warpTiles<2>(a.pi_part, t.x, t.y, lane, ops, out);
-    if (lane == 0) {
-        a.ps[l].s2 = out[0];
-        a.ps[l].nrm = sqrt(out[1]);
-    }
+constexpr int kPowerChunk = 16;  // iterations per graph launch (even: packPowerChunkEnd)
+
+// Residual of a chunk's iteration `it` from its partials, over one warp, and
+// whether it ends LP l's power iteration.
+__device__ __forceinline__ bool packPowerEnds(const PackArgs& a, int l, int4 lp, int it, int lane, double& resid) {
+    const double* part = a.pi_rpart + static_cast<size_t>(it & 1) * a.nct;
+    double acc = 0.0;
+    for (int k = lane; k < lp.y; k += 32) acc += part[lp.x + k];
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+    resid = sqrt(acc);
+    const PowerState& p = a.ps[l];
+    return p.nrmv[it & 1] < 1e-15 || resid < a.sv_tol * fabs(p.s2v[it & 1]) || p.iter + it + 1 >= a.sv_max_iter;
 }
 
-__global__ void __launch_bounds__(kBlock) packPowerNormalize(PackArgs a) {
+// x = x_n / ||x_n|| of a chunk's iteration `it` over a tile, and its residual
+// partial.  Every block sums its LP's dot partials for itself, in their fixed
+// order, and the residual partials of the iteration before, which may have ended
+// it all: as in the single-LP engine, without two one-warp launches in between.
+__global__ void __launch_bounds__(kBlock) packPowerNormalize(PackArgs a, int it) {
     const int tile = blockIdx.x;
     const int4 t = a.ctinfo[tile];
-    const PowerState& ps = a.ps[t.x];
-    if (ps.done) return;
-    const double s2 = ps.s2, nrm = ps.nrm;
+    const int l = t.x;
+    __shared__ int done, ends;
+    __shared__ double dots[2], resid;
+    const int warp = static_cast<int>(threadIdx.x) >> 5, lane = static_cast<int>(threadIdx.x) & 31;
+    const int4 lp = a.lpt[l];
+    // read once per block: the LP's first block may set it while others start
+    if (threadIdx.x == 0) done = a.ps[l].done;
+    if (warp == 0) {
+        const int ops[2] = {OP_SUM, OP_SUM};
+        double out[2];
+        warpTiles<2>(a.pi_part, lp.x, lp.y, lane, ops, out);
+        if (lane == 0) {
+            dots[0] = out[0];
+            dots[1] = sqrt(out[1]);
+        }
+    } else if (warp == 1) {
+        double r = 0.0;
+        const bool e = it > 0 && packPowerEnds(a, l, lp, it - 1, lane, r);
+        if (lane == 0) {
+            ends = e;
+            resid = r;
+        }
+    }
+    __syncthreads();
+    if (done) return;
+    const bool first = tile == lp.x && threadIdx.x == 0;
+    if (ends) {
+        if (first) {
+            PowerState& p = a.ps[l];
+            p.s2 = p.s2v[(it - 1) & 1];
+            p.resid = resid;
+            p.done = 1;
+            atomicAdd(a.counters, 1);
+        }
+        return;
+    }
+    const double s2 = dots[0], nrm = dots[1];
     double acc[1] = {0.0};
     for (int j = t.z + threadIdx.x; j < t.w; j += kBlock) {
         const double xn = a.pi_xn[j];
@@ -651,23 +690,27 @@ __global__ void __launch_bounds__(kBlock) packPowerNormalize(PackArgs a) {
         if (nrm >= 1e-15) a.pi_x[j] = xn / nrm;
     }
     const int ops[1] = {OP_SUM};
-    blockReduceSlots<1>(acc, ops, a.pi_part + static_cast<size_t>(tile) * 2);
+    blockReduceSlots<1>(acc, ops, a.pi_rpart + static_cast<size_t>(it & 1) * a.nct + tile);
+    if (first) {
+        a.ps[l].s2v[it & 1] = s2;
+        a.ps[l].nrmv[it & 1] = nrm;
+    }
 }
 
-__global__ void __launch_bounds__(32 * kCtlWarps) packPowerFinish2(PackArgs a) {
+// The end of a chunk of `its` iterations: the verdict on the last one.
+__global__ void __launch_bounds__(32 * kCtlWarps) packPowerChunkEnd(PackArgs a, int its) {
     const int l = blockIdx.x * kCtlWarps + static_cast<int>(threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (l >= a.L || a.ps[l].done) return;
-    const int4 t = a.lpt[l];
-    double acc = 0.0;
-    for (int k = lane; k < t.y; k += 32) acc += a.pi_part[static_cast<size_t>(t.x + k) * 2];
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+    double resid;
+    const bool ends = packPowerEnds(a, l, a.lpt[l], its - 1, lane, resid);
+    __syncwarp();
     if (lane == 0) {
         PowerState& p = a.ps[l];
-        p.resid = sqrt(acc);
-        p.iter += 1;
-        if (p.nrm < 1e-15 || p.resid < a.sv_tol * fabs(p.s2) || p.iter >= a.sv_max_iter) {
+        p.s2 = p.s2v[(its - 1) & 1];
+        p.resid = resid;
+        p.iter += its;
+        if (ends) {
             p.done = 1;
             atomicAdd(a.counters, 1);
         }
@@ -753,7 +796,7 @@ size_t itemBytes(const Item& it, bool mixed) {
     b += n * (32 + 40 + 8 + 24 + 24) + m * (32 + 32 + 8 + 16 + 8);     // packs, checks, FP64 iterates, power
     if (mixed) b += n * (16 + 12) + m * (16 + 8);
     b += static_cast<size_t>(it.cols.entries + it.rows.entries) * (4 + 8 + (mixed ? 4 : 0)) + (m + n) / 4;
-    b += static_cast<size_t>(it.nct) * (16 + 4 + 8 * kColSlots + 16) + static_cast<size_t>(it.nrt) * (16 + 4 + 8 * kRowSlots);
+    b += static_cast<size_t>(it.nct) * (16 + 4 + 8 * kColSlots + 32) + static_cast<size_t>(it.nrt) * (16 + 4 + 8 * kRowSlots);
     b += sizeof(DevState) + sizeof(DevConst) + sizeof(PowerState) + 32;
     b += n * (16 + 2 + (mixed ? 8 : 0)) + m * (16 + 4) + sizeof(LinkLp);  // linked cycle: cells, units
     return b;
@@ -997,7 +1040,7 @@ struct Pack {
         iter_end = o;
         o_piy = take(8 * m);
         o_pixn = take(8 * n);
-        o_pipart = take(16 * static_cast<size_t>(nct));
+        o_pipart = take(32 * static_cast<size_t>(nct));
         o_pcols = take(8 * kColSlots * static_cast<size_t>(nct));
         o_prows = take(8 * kRowSlots * static_cast<size_t>(nrt));
         o_clist = take(4 * static_cast<size_t>(nct));
@@ -1105,6 +1148,7 @@ struct Pack {
         a.pi_y = P<double>(o_piy);
         a.pi_xn = P<double>(o_pixn);
         a.pi_part = P<double>(o_pipart);
+        a.pi_rpart = a.pi_part + 2 * static_cast<size_t>(nct);
         a.L = L;
         a.nct = nct;
         a.nrt = nrt;
@@ -1321,19 +1365,19 @@ struct Pack {
         const PackArgs& a = args;
         for (int it = 0; it < chunk; ++it) {
             for (const Launch& c : cls_r) {
-                PDLPX_G_SWITCH(checkGroup(c.shape), (packPowerA<GG><<<c.count, kBlock, 0, s>>>(a, c.tile0)));
+                const int passes = tileRows(c.shape) * checkGroup(c.shape) / kBlock;
+                PDLPX_G_SWITCH(checkGroup(c.shape), (packPowerA<GG><<<c.count * passes, kBlock, 0, s>>>(a, c.tile0, passes)));
                 ++n;
             }
             for (const Launch& c : cls_c) {
                 PDLPX_G_SWITCH(checkGroup(c.shape), (packPowerAt<GG><<<c.count, kBlock, 0, s>>>(a, c.tile0)));
                 ++n;
             }
-            packPowerFinish1<<<(L + kCtlWarps - 1) / kCtlWarps, 32 * kCtlWarps, 0, s>>>(a);
-            packPowerNormalize<<<nct, kBlock, 0, s>>>(a);
-            packPowerFinish2<<<(L + kCtlWarps - 1) / kCtlWarps, 32 * kCtlWarps, 0, s>>>(a);
-            n += 3;
+            packPowerNormalize<<<nct, kBlock, 0, s>>>(a, it);
+            ++n;
         }
-        return n;
+        packPowerChunkEnd<<<(L + kCtlWarps - 1) / kCtlWarps, 32 * kCtlWarps, 0, s>>>(a, chunk);
+        return n + 1;
     }
 };
 
@@ -1727,7 +1771,7 @@ int32_t solvePack(Pack& pk, const pdlpx_options& o, std::chrono::steady_clock::t
         cudaGraph_t graph = nullptr;
         PDLPX_BCK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
         if (power)
-            count = pk.launchPower(8);
+            count = pk.launchPower(kPowerChunk);
         else if (&g == &pk.lcycle)
             count = pk.launchLinked(o.termination_eval_frequency, sms) + pk.launchCycle(o.termination_eval_frequency, false);
         else
@@ -1744,7 +1788,7 @@ int32_t solvePack(Pack& pk, const pdlpx_options& o, std::chrono::steady_clock::t
     if (o.sv_max_iter > 0) {
         int32_t rc = capture(pk.power, pk.power_launches, true);
         if (rc != PDLPX_OK) return rc;
-        for (int guard = 0; guard < 2 + o.sv_max_iter / 8; ++guard) {
+        for (int guard = 0; guard < 2 + o.sv_max_iter / kPowerChunk; ++guard) {
             PDLPX_BCK(cudaGraphLaunch(pk.power, s));
             launches += pk.power_launches;
             PDLPX_BCK(cudaMemcpyAsync(h_small, pk.args.counters, 4, cudaMemcpyDeviceToHost, s));
