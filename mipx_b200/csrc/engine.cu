@@ -540,6 +540,7 @@ struct DeviceLp {
     // step shapes shapeLD / shapeLP; the other rows use gA / gAT, shapeD / shapeP.
     int nlD = 0, nlP = 0, gLA = 1, gLAT = 1, shapeLD = 0, shapeLP = 0;
     int64_t zlD = 0, zlP = 0;  // entries of the long rows
+    int32_t longest = 0;       // entries of the longest of them
     // hot prefixes: the primal step's gathers of y[0, hotP) and the dual step's
     // of x[0, hotD) are served from shared memory (0: off); the launch caps
     // them at what one block's shared memory holds
@@ -600,7 +601,9 @@ struct DeviceLp {
     DevState* st = nullptr;
     DevConst* dc = nullptr;
     PowerState* ps = nullptr;
-    DevState* h_st = nullptr;    // pinned mirror
+    StateBlock* h_sb = nullptr;  // two pinned mirrors of the state block, for cycles in turn
+    DevState* h_st = nullptr;    // h_sb[0].st
+    cudaEvent_t copied[2] = {nullptr, nullptr};  // the mirror's copy is done
     PowerState* h_ps = nullptr;  // pinned mirror
 
     // linked restart cycle (linked.cuh): whether it runs the steps, lanes per
@@ -627,7 +630,9 @@ struct DeviceLp {
                 if (e) cudaEventDestroy(e);
         if (power) cudaGraphExecDestroy(power);
         if (arena) cudaFree(arena);
-        if (h_st) cudaFreeHost(h_st);
+        if (h_sb) cudaFreeHost(h_sb);
+        for (auto& e : copied)
+            if (e) cudaEventDestroy(e);
         if (h_ps) cudaFreeHost(h_ps);
         if (stream) cudaStreamDestroy(stream);
     }
@@ -984,8 +989,11 @@ LinkSide<T> linkSide(const DeviceLp& d, const IterArgs<T>& ia, bool primal) {
 //    that 2 (20,000 x 50,000 12.3 against 14.1: more warps than an SM holds).
 //    Columns of up to 3 entries take one lane (transportation 30 x 40: 2.6
 //    against 2.8), long ones 8.
-//  * long rows beside sliced ELL: power law 2,000 x 8,000 20.4 -> 10.8, 8,000 x
-//    32,000 (321k entries) 37 -> 30, 25,000 x 100,000 (1.0M) 37 -> 50: to 400k.
+//  * long rows beside sliced ELL (power law, launches with long and short columns
+//    in one): columns of up to 500 entries at 1,000 x 4,000 14.9 -> 6.9, 4,000 x
+//    16,000 16.0 -> 13.4, 8,000 x 32,000 (317k entries) 17.7 -> 15.8, up to 1,000
+//    at 2,000 x 8,000 16.0 -> 9.5, but up to 2,000 at 4,000 x 16,000 16.4 -> 19.1
+//    (one warp sums a long row): to 350k entries and rows of 1,000.
 //  * a CSR side: transportation 97 x 131 (25k entries) 5.7 -> 3.9, 150 x 150 5.7 ->
 //    5.4, 200 x 200 (80k) 5.9 -> 5.8, 300 x 300 7.2 -> 7.8: to 60k.
 // Options that pin a launch shape keep the launches.
@@ -994,7 +1002,8 @@ bool linkable(const DeviceLp& d, const pdlpx_options& o) {
     if (d.lt_C > 0 || o.hot_cache > 0) return false;
     if (o.shape_primal > 0 || o.shape_dual > 0 || o.spmv_group_a > 0 || o.spmv_group_at > 0) return false;
     const bool csr = !isSell(d.shapeP) || !isSell(d.shapeD);
-    return d.nnz <= (csr ? 60000 : (d.nlP > 0 || d.nlD > 0) ? 400000 : 600000);
+    if (d.longest > 1000) return false;
+    return d.nnz <= (csr ? 60000 : (d.nlP > 0 || d.nlD > 0) ? 350000 : 600000);
 }
 void planLinked(DeviceLp& d) {
     // rowDotU with two sums per lane (the autotuner may pick it) has no linked form
@@ -1538,6 +1547,7 @@ static int32_t buildDevice(std::unique_ptr<DeviceLp>& dp, const ScaledLp& sc_in,
     const int64_t zlD = d.nlD > 0 ? sc.a.ptr[d.nlD] : 0, zlP = d.nlP > 0 ? sc.at.ptr[d.nlP] : 0;
     d.zlD = zlD;
     d.zlP = zlP;
+    d.longest = std::max(d.nlD > 0 ? sc.a.ptr[1] : 0, d.nlP > 0 ? sc.at.ptr[1] : 0);  // the longest come first
     LongTilesHost ltH;
     // automatic: when the long columns hold at least 1.5 times as many entries
     // per SM as a chunk has rows (each tile's copy of y then serves >= 1.5
@@ -1652,7 +1662,9 @@ static int32_t buildDevice(std::unique_ptr<DeviceLp>& dp, const ScaledLp& sc_in,
     d.arena_bytes = off;
     const auto tb1 = std::chrono::steady_clock::now();
     PDLPX_CK(cudaMalloc(reinterpret_cast<void**>(&d.arena), d.arena_bytes));
-    PDLPX_CK(cudaMallocHost(reinterpret_cast<void**>(&d.h_st), sizeof(StateBlock)));
+    PDLPX_CK(cudaMallocHost(reinterpret_cast<void**>(&d.h_sb), 2 * sizeof(StateBlock)));
+    d.h_st = &d.h_sb[0].st;
+    for (auto& e : d.copied) PDLPX_CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     PDLPX_CK(cudaMallocHost(reinterpret_cast<void**>(&d.h_ps), sizeof(PowerState)));
     char* b = d.arena;
     d.a_ptr = reinterpret_cast<int*>(b + o_a_ptr);
@@ -2405,41 +2417,75 @@ int32_t Engine::solveDevice(pdlpx_result* out) {
         step_ms_[p][0] = step_ms_[p][1] = 0.0;
         step_samples_[p] = 0;
     }
+    // A linked cycle is short beside the way to the host and back (25 us of 400-600),
+    // so the next one is queued before the state of the one at hand is read; once
+    // the solve has ended, what is queued returns at once.
+    struct Queued {
+        int prec, link;
+    } queue[2] = {};
+    int head = 0, queued = 0;
+    for (int k = 0; k < 2; ++k) {
+        d.h_sb[k].st = st0;
+        d.h_sb[k].link_err = 0;
+    }
+    struct Drain {  // whichever way this returns, nothing queued writes the mirrors later
+        cudaStream_t s;
+        ~Drain() { cudaStreamSynchronize(s); }
+    } drain{s};
+    auto enqueue = [&](int link) -> int32_t {
+        const int32_t rc = ensureCycle(prec, link);
+        if (rc != PDLPX_OK) return rc;
+        const int slot = (head + queued) & 1;
+        PDLPX_CK(cudaGraphLaunch(d.cycle[prec][link], s));
+        launches += d.launches_cycle[prec][link];
+        PDLPX_CK(cudaMemcpyAsync(&d.h_sb[slot], d.st, sizeof(StateBlock), cudaMemcpyDeviceToHost, s));
+        PDLPX_CK(cudaEventRecord(d.copied[slot], s));
+        queue[slot] = Queued{prec, link};
+        ++queued;
+        return PDLPX_OK;
+    };
     while (true) {
         if (timeUp(t0, opt_.max_solve_seconds)) break;
         if (stopRequested()) {
             stopped = true;
             break;
         }
-        const int link = d.linked && link_share.fits() ? 1 : 0;
-        const int32_t rc = ensureCycle(prec, link);
-        if (rc != PDLPX_OK) return rc;
-        PDLPX_CK(cudaGraphLaunch(d.cycle[prec][link], s));
-        launches += d.launches_cycle[prec][link];
-        PDLPX_CK(cudaMemcpyAsync(d.h_st, d.st, sizeof(StateBlock), cudaMemcpyDeviceToHost, s));
-        PDLPX_CK(cudaStreamSynchronize(s));
-        const DevState& h = *d.h_st;
-        if (reinterpret_cast<const StateBlock*>(d.h_st)->link_err != 0) {
+        const int want = d.linked && link_share.fits() ? 1 : 0;
+        if (queued == 0) {
+            const int32_t rc = enqueue(want);
+            if (rc != PDLPX_OK) return rc;
+        }
+        if (want && queued == 1 && queue[head].link) {
+            const int32_t rc = enqueue(1);
+            if (rc != PDLPX_OK) return rc;
+        }
+        PDLPX_CK(cudaEventSynchronize(d.copied[head]));
+        const StateBlock& block = d.h_sb[head];
+        const DevState& h = block.st;
+        const int link = queue[head].link, ran = queue[head].prec;
+        head ^= 1;
+        --queued;
+        if (block.link_err != 0) {
             err = "linked cycle: a wait ran out of polls";
             return PDLPX_E_TIMEOUT;
         }
         if (link) {
-            const LinkTime& q = reinterpret_cast<const StateBlock*>(d.h_st)->lt;
+            const LinkTime& q = block.lt;
             const double clk = static_cast<double>(q.primal_clk + q.dual_clk);
             if (h.total > prev_total && q.iters > 0 && clk > 0.0) {
                 const double ms = 1e-6 * static_cast<double>(q.ns) / q.iters;
-                step_ms_[prec][0] += ms * static_cast<double>(q.primal_clk) / clk;
-                step_ms_[prec][1] += ms * static_cast<double>(q.dual_clk) / clk;
-                ++step_samples_[prec];
+                step_ms_[ran][0] += ms * static_cast<double>(q.primal_clk) / clk;
+                step_ms_[ran][1] += ms * static_cast<double>(q.dual_clk) / clk;
+                ++step_samples_[ran];
             }
         } else if (h.total - prev_total >= d.kev_iter) {
             // the timed iteration ran in full: read the step kernels' events of this cycle
             float a = 0.0f, b = 0.0f;
-            if (cudaEventElapsedTime(&a, d.kev[prec][0], d.kev[prec][1]) == cudaSuccess &&
-                cudaEventElapsedTime(&b, d.kev[prec][1], d.kev[prec][2]) == cudaSuccess) {
-                step_ms_[prec][0] += a;
-                step_ms_[prec][1] += b;
-                ++step_samples_[prec];
+            if (cudaEventElapsedTime(&a, d.kev[ran][0], d.kev[ran][1]) == cudaSuccess &&
+                cudaEventElapsedTime(&b, d.kev[ran][1], d.kev[ran][2]) == cudaSuccess) {
+                step_ms_[ran][0] += a;
+                step_ms_[ran][1] += b;
+                ++step_samples_[ran];
             } else {
                 (void)cudaGetLastError();
             }
@@ -2462,7 +2508,14 @@ int32_t Engine::solveDevice(pdlpx_result* out) {
     float ms = 0.0f;
     cudaEventElapsedTime(&ms, ev0, ev1);
 
-    const DevState fin = *d.h_st;
+    // ev1 waited for what was queued: the last copy is the final state (no cycle: the
+    // initial one)
+    const StateBlock& last_block = d.h_sb[(head + queued + 1) & 1];
+    const DevState fin = last_block.st;
+    if (last_block.link_err != 0) {
+        err = "linked cycle: a wait ran out of polls";
+        return PDLPX_E_TIMEOUT;
+    }
     int32_t status;
     if (fin.done) {
         status = fin.status;
