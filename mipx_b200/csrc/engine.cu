@@ -396,8 +396,8 @@ __global__ void __launch_bounds__(kBlock, sellMinBlocks<float, true>())
 }
 
 // ---- linked restart cycle (linked.cuh) ------------------------------------------
-// 16 warps at 128 registers; with CSR rows, whose eight sums per lane would
-// spill there, 8 warps.
+// 16 warps at 128 registers; with CSR rows, whose eight cells and sums per lane
+// would spill there, 8 warps.
 constexpr int linkThreads(bool csr) { return csr ? 256 : 512; }
 template <int LP, int LD, bool CSR, class T>
 __global__ void __launch_bounds__(linkThreads(CSR), 1) linkedSteps(LinkArgs<T> a) {
@@ -994,8 +994,8 @@ LinkSide<T> linkSide(const DeviceLp& d, const IterArgs<T>& ia, bool primal) {
 //    16,000 16.0 -> 13.4, 8,000 x 32,000 (317k entries) 17.7 -> 15.8, up to 1,000
 //    at 2,000 x 8,000 16.0 -> 9.5, but up to 2,000 at 4,000 x 16,000 16.4 -> 19.1
 //    (one warp sums a long row): to 350k entries and rows of 1,000.
-//  * a CSR side: transportation 97 x 131 (25k entries) 5.7 -> 3.9, 150 x 150 5.7 ->
-//    5.4, 200 x 200 (80k) 5.9 -> 5.8, 300 x 300 7.2 -> 7.8: to 60k.
+//  * a CSR side: transportation 97 x 131 (25k entries) 5.7 -> 3.3, 150 x 150 5.7 ->
+//    4.7, 200 x 200 (80k) 5.5 -> 5.4, 250 x 250 5.8 -> 6.4: to 90k.
 // Options that pin a launch shape keep the launches.
 bool linkCsr(const DeviceLp& d) { return !isSell(d.shapeP) || !isSell(d.shapeD) || d.nlP > 0 || d.nlD > 0; }
 bool linkable(const DeviceLp& d, const pdlpx_options& o) {
@@ -1003,7 +1003,7 @@ bool linkable(const DeviceLp& d, const pdlpx_options& o) {
     if (o.shape_primal > 0 || o.shape_dual > 0 || o.spmv_group_a > 0 || o.spmv_group_at > 0) return false;
     const bool csr = !isSell(d.shapeP) || !isSell(d.shapeD);
     if (d.longest > 1000) return false;
-    return d.nnz <= (csr ? 60000 : (d.nlP > 0 || d.nlD > 0) ? 350000 : 600000);
+    return d.nnz <= (csr ? 90000 : (d.nlP > 0 || d.nlD > 0) ? 350000 : 600000);
 }
 void planLinked(DeviceLp& d) {
     // rowDotU with two sums per lane (the autotuner may pick it) has no linked form

@@ -44,6 +44,11 @@ namespace pdlpx {
 constexpr int kLinkPolls = 1 << 22;  // ~2 s of L2 round trips
 
 constexpr int kLinkU = 4;  // cells per lane per round
+// Sleep between polls (ns) beside CSR rows: their LPs have few rows or columns that
+// everything gathers, and warps polling the same few lines of L2 hold up the
+// stores to them.  Transportation 97 x 131 3.80 -> 3.30 us per iteration, 150 x 150
+// 5.71 -> 4.72 (B200); LPs without such rows lose 0-4 % by it.
+constexpr int kLinkNap = 80;
 
 // Device time of the last cycle: all of it (globaltimer), and the SM clocks that
 // a row's warp waited for and summed new x (the primal half-steps) and a
@@ -156,20 +161,22 @@ struct LinkReg<float> {
 // The cells x[c[u]] of iteration `tag`, loaded until all of the warp's are
 // there; entries with value 0 are not waited for and give 0.  The warp polls
 // together: with lanes that leave the loop one by one the same kernel took 5-10
-// times as long.  False when the wait ran out.
-template <class V, class X>
-__device__ __forceinline__ bool linkGather(const LinkCell<X>* __restrict__ x, const int (&c)[kLinkU],
-                                           const V (&v)[kLinkU], unsigned tag, X (&g)[kLinkU], int* err) {
-    LinkReg<X> r[kLinkU];
+// times as long.  NAP: nanoseconds of sleep between polls.  False when the wait
+// ran out.
+template <int U, int NAP, class V, class X>
+__device__ __forceinline__ bool linkGather(const LinkCell<X>* __restrict__ x, const int (&c)[U], const V (&v)[U],
+                                           unsigned tag, X (&g)[U], int* err) {
+    LinkReg<X> r[U];
 #pragma unroll
-    for (int u = 0; u < kLinkU; ++u) r[u].set(v[u] == V(0) ? tag : ~tag);
+    for (int u = 0; u < U; ++u) r[u].set(v[u] == V(0) ? tag : ~tag);
     for (int polls = 0;;) {
 #pragma unroll
-        for (int u = 0; u < kLinkU; ++u) r[u].load(x + c[u], tag);
+        for (int u = 0; u < U; ++u) r[u].load(x + c[u], tag);
         bool ready = true;
 #pragma unroll
-        for (int u = 0; u < kLinkU; ++u) ready = ready && r[u].ready(tag);
+        for (int u = 0; u < U; ++u) ready = ready && r[u].ready(tag);
         if (__all_sync(0xffffffffu, ready)) break;
+        if constexpr (NAP > 0) __nanosleep(NAP);
         if ((++polls & 1023) == 0) {
             const bool out = polls >= kLinkPolls || *reinterpret_cast<volatile int*>(err) != 0;
             if (__any_sync(0xffffffffu, out)) {
@@ -179,14 +186,14 @@ __device__ __forceinline__ bool linkGather(const LinkCell<X>* __restrict__ x, co
         }
     }
 #pragma unroll
-    for (int u = 0; u < kLinkU; ++u) g[u] = r[u].value();
+    for (int u = 0; u < U; ++u) g[u] = r[u].value();
     return true;
 }
 
 // One slice's rows with L lanes each (32 / L rows per warp): a lane gathers
 // every L-th entry of row r of the slice, and the entries go into the sum one by
 // one in sellDot's order, handed round by shuffles.
-template <int L, class V, class X>
+template <int L, int NAP = 0, class V, class X>
 __device__ __forceinline__ double linkSellDot(const int* __restrict__ idx, const V* __restrict__ val, int2 h, int r,
                                               int lane, const LinkCell<X>* x, unsigned tag, int* err, bool& ok) {
     const int q = lane % L;
@@ -204,7 +211,7 @@ __device__ __forceinline__ double linkSellDot(const int* __restrict__ idx, const
             c[u] = in ? __ldg(ip + k * kSlice) : 0;
             v[u] = in ? __ldg(vp + k * kSlice) : V(0);
         }
-        ok = linkGather(x, c, v, tag, g, err) && ok;
+        ok = linkGather<kLinkU, NAP>(x, c, v, tag, g, err) && ok;
 #pragma unroll
         for (int u = 0; u < kLinkU; ++u) {
             if (k0 + u * L >= h.y) break;  // the same in every lane
@@ -231,24 +238,23 @@ __device__ __forceinline__ double linkLaneSum(int b, int e, int first, int G, co
     double s[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) s[u] = 0.0;
-    const int rounds = __reduce_max_sync(0xffffffffu, (e - b + U * G - 1) / (U * G));
-    for (int k0 = b + first, q = 0; q < rounds; ++q, k0 += U * G) {
+    // eight cells in flight: two of rowDotU's rounds of four, or one of eight
+    constexpr int W = 8;
+    const int rounds = __reduce_max_sync(0xffffffffu, (e - b + W * G - 1) / (W * G));
+    for (int k0 = b + first, q = 0; q < rounds; ++q, k0 += W * G) {
+        int c[W];
+        V v[W];
+        X g[W];
 #pragma unroll
-        for (int w = 0; w < U; w += kLinkU) {
-            int c[kLinkU];
-            V v[kLinkU];
-            X g[kLinkU];
-#pragma unroll
-            for (int u = 0; u < kLinkU; ++u) {
-                const int k = k0 + (w + u) * G;
-                const bool in = k < e;
-                c[u] = in ? __ldg(idx + k) : 0;
-                v[u] = in ? __ldg(val + k) : V(0);
-            }
-            ok = linkGather(x, c, v, tag, g, err) && ok;
-#pragma unroll
-            for (int u = 0; u < kLinkU; ++u) s[w + u] += static_cast<double>(v[u]) * static_cast<double>(g[u]);
+        for (int u = 0; u < W; ++u) {
+            const int k = k0 + u * G;
+            const bool in = k < e;
+            c[u] = in ? __ldg(idx + k) : 0;
+            v[u] = in ? __ldg(val + k) : V(0);
         }
+        ok = linkGather<W, kLinkNap>(x, c, v, tag, g, err) && ok;
+#pragma unroll
+        for (int u = 0; u < W; ++u) s[u % U] += static_cast<double>(v[u]) * static_cast<double>(g[u]);
     }
     double t = s[0];
 #pragma unroll
@@ -307,7 +313,7 @@ __device__ __forceinline__ double linkUnitDot(const LinkSide<T>& a, int u, int l
                                               int* err, bool& ok) {
     if (!CSR || (u >= a.nl && a.lanes == 0)) {
         const int v = u - a.nl;
-        return linkSellDot<L>(a.idx, a.val, __ldg(a.hdr + v / L), v % L * (32 / L) + lane / L, lane, x, tag, err, ok);
+        return linkSellDot<L, CSR ? kLinkNap : 0>(a.idx, a.val, __ldg(a.hdr + v / L), v % L * (32 / L) + lane / L, lane, x, tag, err, ok);
     }
     const bool lng = u < a.nl;
     const int G = lng ? a.llanes : a.lanes, W = lng ? a.lunroll : a.unroll;

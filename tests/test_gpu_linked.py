@@ -76,7 +76,7 @@ def test_empty_rows_and_columns(m, n):
     _same(_holes(m, n, m), SELL, max_iter=1000)
 
 
-@pytest.mark.parametrize("s,d", [(70, 80), (97, 131), (130, 180)])
+@pytest.mark.parametrize("s,d", [(70, 80), (97, 131), (130, 180), (200, 210)])
 @pytest.mark.parametrize("fp32", [False, True])
 def test_csr_rows(s, d, fp32):
     lp, _ = G.transport_lp(s, d, 3)
