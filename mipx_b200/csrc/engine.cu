@@ -27,6 +27,7 @@
 #include "control.cuh"
 #include "linked.cuh"
 #include "shapes.cuh"
+#include "tiny.cuh"
 
 namespace pdlpx {
 
@@ -611,6 +612,8 @@ struct DeviceLp {
     bool linked = false;
     int link_lanes = 4;
     int link_warps = 0;  // of its grid per SM
+    int tiny = 0;        // one block runs it (tiny.cuh): 1 short columns, 2 short rows
+    int sell_max[2] = {0, 0};  // most entries of a sliced-ELL column / row
     void *link_x = nullptr, *link_y = nullptr;  // cells (null: the launches run)
 
     // [FP32 / FP64][step launches / linked]
@@ -996,6 +999,9 @@ LinkSide<T> linkSide(const DeviceLp& d, const IterArgs<T>& ia, bool primal) {
 //    (one warp sums a long row): to 350k entries and rows of 1,000.
 //  * a CSR side: transportation 97 x 131 (25k entries) 5.7 -> 3.3, 150 x 150 5.7 ->
 //    4.7, 200 x 200 (80k) 5.5 -> 5.4, 250 x 250 5.8 -> 6.4: to 90k.
+//  * one block takes an LP whose slices are its warps and whose entries fit their
+//    registers (tiny.cuh): 90 x 250 linked 2.3 -> 1.2.  No block waits on another,
+//    so it needs no share of the SMs (link_warps 0).
 // Options that pin a launch shape keep the launches.
 bool linkCsr(const DeviceLp& d) { return !isSell(d.shapeP) || !isSell(d.shapeD) || d.nlP > 0 || d.nlD > 0; }
 bool linkable(const DeviceLp& d, const pdlpx_options& o) {
@@ -1009,7 +1015,15 @@ void planLinked(DeviceLp& d) {
     // rowDotU with two sums per lane (the autotuner may pick it) has no linked form
     auto supported = [](int shape) { return isSell(shape) || kShapes[shape].U >= kLinkU; };
     d.linked = d.link_x != nullptr && supported(d.shapeP) && supported(d.shapeD);
+    d.tiny = d.link_warps = 0;
     if (!d.linked) return;
+    if (!linkCsr(d) && (d.n + kSlice - 1) / kSlice + (d.m + kSlice - 1) / kSlice <= kTinyWarps) {
+        if (d.sell_max[0] <= kTinyShort && d.sell_max[1] <= kTinyLong)
+            d.tiny = 1;
+        else if (d.sell_max[0] <= kTinyLong && d.sell_max[1] <= kTinyShort)
+            d.tiny = 2;
+    }
+    if (d.tiny != 0) return;
     const double mean = static_cast<double>(d.nnz - d.zlP) / std::max(1, d.n - d.nlP);
     d.link_lanes = mean <= 3.0 ? 1 : mean > 14.0 ? 8 : d.nnz <= 240000 ? 4 : 2;
     const bool csr = linkCsr(d);
@@ -1049,6 +1063,14 @@ cudaError_t launchLinked(const DeviceLp& d, const IterArgs<T>& ia, cudaStream_t 
     a.y = static_cast<LinkCell<T>*>(d.link_y);
     a.err = &reinterpret_cast<StateBlock*>(d.st)->link_err;
     a.time = &reinterpret_cast<StateBlock*>(d.st)->lt;
+    if (d.tiny != 0) {
+        const int threads = 32 * ((d.n + kSlice - 1) / kSlice + (d.m + kSlice - 1) / kSlice);
+        if (d.tiny == 1)
+            tinySteps<kTinyShort, kTinyLong, T><<<1, threads, 0, s>>>(a);
+        else
+            tinySteps<kTinyLong, kTinyShort, T><<<1, threads, 0, s>>>(a);
+        return cudaGetLastError();
+    }
     if (linkCsr(d))
         return d.link_lanes == 1 ? launchLinkedAs<1, 8, true, T>(d, a, s) : launchLinkedAs<4, 8, true, T>(d, a, s);
     switch (d.link_lanes) {
@@ -1538,6 +1560,8 @@ static int32_t buildDevice(std::unique_ptr<DeviceLp>& dp, const ScaledLp& sc_in,
     SellHost hsP, hsD;
     if (sellP && !buildSell(sc.at, d.nlP, hsP)) sellP = false;
     if (sellD && !buildSell(sc.a, d.nlD, hsD)) sellD = false;
+    for (const int2& h : hsP.hdr) d.sell_max[0] = std::max(d.sell_max[0], h.y);
+    for (const int2& h : hsD.hdr) d.sell_max[1] = std::max(d.sell_max[1], h.y);
     const auto tbs = std::chrono::steady_clock::now();
     d.m = sc.a.rows;
     d.n = sc.a.cols;
@@ -2450,7 +2474,7 @@ int32_t Engine::solveDevice(pdlpx_result* out) {
             stopped = true;
             break;
         }
-        const int want = d.linked && link_share.fits() ? 1 : 0;
+        const int want = d.linked && (d.tiny != 0 || link_share.fits()) ? 1 : 0;
         if (queued == 0) {
             const int32_t rc = enqueue(want);
             if (rc != PDLPX_OK) return rc;

@@ -393,6 +393,14 @@ constexpr StepShape kShapes[] = {
 };
 constexpr int kNumShapes = sizeof(kShapes) / sizeof(kShapes[0]);
 
+// The steps' sums of products are rounded as written here in every kernel: left to
+// itself the compiler fuses one product or the other, or none that it can move out
+// of a loop, by what surrounds them.
+// lam r + (1 - lam) a
+__device__ __forceinline__ double average(double lam, double r, double a) {
+    return __fma_rn(1.0 - lam, a, __dmul_rn(lam, r));
+}
+
 // Values of the Halpern primal step of a column given s = (A^T y_cur)_j:
 // projected gradient step (xh), reflection (xr), averaging with the anchor
 // (returned: the new current x) (pdlp_kernels.cu:46-88).  FP64 arithmetic with
@@ -400,12 +408,12 @@ constexpr int kNumShapes = sizeof(kShapes) / sizeof(kShapes[0]);
 template <class T>
 __device__ __forceinline__ double primalValues(const ColPack<T>& q, double xcd, double xid, double s, double tau,
                                                double lam, double& xh, double& xr) {
-    xh = xcd - tau * (static_cast<double>(q.c) + s);
+    xh = __fma_rn(-tau, static_cast<double>(q.c) + s, xcd);
     const double lb = q.lb, ub = q.ub;
     if (xh < lb) xh = lb;
     if (xh > ub) xh = ub;
     xr = 2.0 * xh - xcd;
-    return lam * xr + (1.0 - lam) * xid;
+    return average(lam, xr, xid);
 }
 
 template <class T>
@@ -426,27 +434,27 @@ template <class T>
 __device__ __forceinline__ double dualValues(const RowPack<T>& q, double ycd, double yid, double s, double step,
                                              double pw, double lam, double& py) {
     const double sig = step * static_cast<double>(q.sigma) * pw;
-    const double v = ycd + sig * s;
+    const double v = __fma_rn(sig, s, ycd);
     const double rl = q.rl, ru = q.ru;
     const int type = static_cast<int>(q.type);
     if (type == 0) {
-        py = v - sig * rl;
+        py = __fma_rn(-sig, rl, v);
     } else if (type == 1) {
-        py = v - sig * ru;
+        py = __fma_rn(-sig, ru, v);
         if (py < 0.0) py = 0.0;
     } else if (type == 2) {
-        py = v - sig * rl;
+        py = __fma_rn(-sig, rl, v);
         if (py > 0.0) py = 0.0;
     } else {
-        if (v >= sig * ru)
-            py = v - sig * ru;
-        else if (v <= sig * rl)
-            py = v - sig * rl;
+        if (v >= __dmul_rn(sig, ru))
+            py = __dsub_rn(v, __dmul_rn(sig, ru));
+        else if (v <= __dmul_rn(sig, rl))
+            py = __dsub_rn(v, __dmul_rn(sig, rl));
         else
             py = 0.0;
     }
     const double yr = 2.0 * py - ycd;
-    return lam * yr + (1.0 - lam) * yid;
+    return average(lam, yr, yid);
 }
 
 template <class T>

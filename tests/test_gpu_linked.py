@@ -71,6 +71,22 @@ def test_sliced_ell(m, n, lo, hi, precision):
     _same(lp, SELL, precision=precision, fp64_switch=precision == Precision.FP64, max_iter=1500)
 
 
+# one block: 12 slices and 13, up to 16 entries on one side and 40 on the other
+# (and one more), either side the short one, rows with two finite sides
+@pytest.mark.parametrize("m,n,lo,hi", [(32, 352, 1, 3), (33, 352, 1, 3), (352, 32, 20, 32), (240, 120, 8, 30),
+                                       (90, 250, 4, 16), (90, 250, 4, 17), (60, 150, 12, 16), (41, 41, 40, 41)])
+@pytest.mark.parametrize("precision", [Precision.FP64, Precision.Mixed])
+@pytest.mark.parametrize("ranged", [False, True])
+def test_one_block(m, n, lo, hi, precision, ranged):
+    lp, _ = G.random_lp(m, n, lo, hi, 7 + m)
+    if ranged:
+        hi_side = np.where(np.isfinite(lp.row_upper), lp.row_upper, lp.row_lower + 1.0)
+        lo_side = np.where(np.isfinite(lp.row_lower), lp.row_lower, lp.row_upper - 1.0)
+        lp.row_lower, lp.row_upper = np.minimum(lo_side, hi_side - 0.5), hi_side
+    _same(lp, SELL, precision=precision, max_iter=1500)
+    _same(lp, SELL, precision=precision, fp64_switch=False, max_iter=450)
+
+
 @pytest.mark.parametrize("m,n", [(5, 40), (64, 50), (700, 900)])
 def test_empty_rows_and_columns(m, n):
     _same(_holes(m, n, m), SELL, max_iter=1000)
