@@ -17,8 +17,8 @@
 // The primal step stores c .* x_refl and the dual step r .* y_cur next to the
 // iterates, so the gathers need no scale factor.  Rows an LP appends after the
 // base rows ("cut rows") are its own CSR rows, handled by a warp per row in the
-// dual step and, for the primal step, by a per-column list of the appended
-// entries of every LP.
+// dual step and, for the primal step, by per-column lists of the appended
+// entries, in lane order, that the warp or every lane for itself walks.
 //
 // Iterates are FP64 throughout (the shared matrix is read once per iteration,
 // so the per-LP vectors are the traffic); per-LP DevState / DevConst and the
