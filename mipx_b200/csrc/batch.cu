@@ -638,50 +638,43 @@ __device__ __forceinline__ bool packPowerEnds(const PackArgs& a, int l, int4 lp,
     return p.nrmv[it & 1] < 1e-15 || resid < a.sv_tol * fabs(p.s2v[it & 1]) || p.iter + it + 1 >= a.sv_max_iter;
 }
 
+// The LPs' dot sums of a chunk's iteration `it` and the verdict on the one before,
+// a warp per LP: a launch of its own, because with every block of the normalisation
+// doing both for itself (as in the single-LP engine) 10,000 blocks each walked their
+// LP's partials.  Power phase of a batch in ms (B200; two one-warp launches, sums in
+// every block, this): 12 LPs 13.2, 10.1, 9.9; 64 33.3, 32.6, 24.7; 128 43.4, 45.3,
+// 37.2; 256 89.5, 128, 83.3; 512 131, 232, 120.
+__global__ void __launch_bounds__(32 * kCtlWarps) packPowerSums(PackArgs a, int it) {
+    const int l = blockIdx.x * kCtlWarps + static_cast<int>(threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    if (l >= a.L || a.ps[l].done) return;
+    const int4 lp = a.lpt[l];
+    const int ops[2] = {OP_SUM, OP_SUM};
+    double out[2], resid = 0.0;
+    warpTiles<2>(a.pi_part, lp.x, lp.y, lane, ops, out);
+    const bool ends = it > 0 && packPowerEnds(a, l, lp, it - 1, lane, resid);
+    __syncwarp();
+    if (lane != 0) return;
+    PowerState& p = a.ps[l];
+    if (ends) {
+        p.s2 = p.s2v[(it - 1) & 1];
+        p.resid = resid;
+        p.done = 1;
+        atomicAdd(a.counters, 1);
+    } else {
+        p.s2v[it & 1] = out[0];
+        p.nrmv[it & 1] = sqrt(out[1]);
+    }
+}
+
 // x = x_n / ||x_n|| of a chunk's iteration `it` over a tile, and its residual
-// partial.  Every block sums its LP's dot partials for itself, in their fixed
-// order, and the residual partials of the iteration before, which may have ended
-// it all: as in the single-LP engine, without two one-warp launches in between.
+// partial.
 __global__ void __launch_bounds__(kBlock) packPowerNormalize(PackArgs a, int it) {
     const int tile = blockIdx.x;
     const int4 t = a.ctinfo[tile];
-    const int l = t.x;
-    __shared__ int done, ends;
-    __shared__ double dots[2], resid;
-    const int warp = static_cast<int>(threadIdx.x) >> 5, lane = static_cast<int>(threadIdx.x) & 31;
-    const int4 lp = a.lpt[l];
-    // read once per block: the LP's first block may set it while others start
-    if (threadIdx.x == 0) done = a.ps[l].done;
-    if (warp == 0) {
-        const int ops[2] = {OP_SUM, OP_SUM};
-        double out[2];
-        warpTiles<2>(a.pi_part, lp.x, lp.y, lane, ops, out);
-        if (lane == 0) {
-            dots[0] = out[0];
-            dots[1] = sqrt(out[1]);
-        }
-    } else if (warp == 1) {
-        double r = 0.0;
-        const bool e = it > 0 && packPowerEnds(a, l, lp, it - 1, lane, r);
-        if (lane == 0) {
-            ends = e;
-            resid = r;
-        }
-    }
-    __syncthreads();
-    if (done) return;
-    const bool first = tile == lp.x && threadIdx.x == 0;
-    if (ends) {
-        if (first) {
-            PowerState& p = a.ps[l];
-            p.s2 = p.s2v[(it - 1) & 1];
-            p.resid = resid;
-            p.done = 1;
-            atomicAdd(a.counters, 1);
-        }
-        return;
-    }
-    const double s2 = dots[0], nrm = dots[1];
+    const PowerState& p = a.ps[t.x];
+    if (p.done) return;
+    const double s2 = p.s2v[it & 1], nrm = p.nrmv[it & 1];
     double acc[1] = {0.0};
     for (int j = t.z + threadIdx.x; j < t.w; j += kBlock) {
         const double xn = a.pi_xn[j];
@@ -691,10 +684,6 @@ __global__ void __launch_bounds__(kBlock) packPowerNormalize(PackArgs a, int it)
     }
     const int ops[1] = {OP_SUM};
     blockReduceSlots<1>(acc, ops, a.pi_rpart + static_cast<size_t>(it & 1) * a.nct + tile);
-    if (first) {
-        a.ps[l].s2v[it & 1] = s2;
-        a.ps[l].nrmv[it & 1] = nrm;
-    }
 }
 
 // The end of a chunk of `its` iterations: the verdict on the last one.
@@ -1373,8 +1362,9 @@ struct Pack {
                 PDLPX_G_SWITCH(checkGroup(c.shape), (packPowerAt<GG><<<c.count, kBlock, 0, s>>>(a, c.tile0)));
                 ++n;
             }
+            packPowerSums<<<(L + kCtlWarps - 1) / kCtlWarps, 32 * kCtlWarps, 0, s>>>(a, it);
             packPowerNormalize<<<nct, kBlock, 0, s>>>(a, it);
-            ++n;
+            n += 2;
         }
         packPowerChunkEnd<<<(L + kCtlWarps - 1) / kCtlWarps, 32 * kCtlWarps, 0, s>>>(a, chunk);
         return n + 1;
