@@ -106,6 +106,7 @@ __device__ __forceinline__ unsigned long long linkWord(unsigned v, unsigned tag)
     asm("mov.b64 %0, {%1, %2};" : "=l"(w) : "r"(v), "r"(tag));
     return w;
 }
+__device__ __forceinline__ unsigned linkTag(unsigned long long w) { return static_cast<unsigned>(w >> 32); }
 __device__ __forceinline__ void linkStore(LinkCell<double>* c, double v, unsigned tag) {
     asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(c),
                  "l"(linkWord(static_cast<unsigned>(__double2loint(v)), tag)),
@@ -116,46 +117,43 @@ __device__ __forceinline__ void linkStore(LinkCell<float>* c, float v, unsigned 
     asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(c), "l"(linkWord(__float_as_uint(v), tag)) : "memory");
 }
 // A cell in registers, loaded again unless it is the wanted one (predicated, so
-// that the loads of a round stay in flight together).
+// that the loads of a round stay in flight together).  A load's elements are the
+// 64-bit words that linkStore writes: only within an element is a value sure to
+// come with its own number -- the elements of a vector load are accesses of their
+// own, in no given order.
 template <class X>
 struct LinkReg;
 template <>
 struct LinkReg<double> {
-    unsigned v0, t0, v1, t1;
-    __device__ __forceinline__ void set(unsigned tag) {
-        v0 = v1 = 0u;
-        t0 = t1 = tag;
-    }
+    unsigned long long w0, w1;
+    __device__ __forceinline__ void set(unsigned tag) { w0 = w1 = linkWord(0u, tag); }
     __device__ __forceinline__ void load(const LinkCell<double>* c, unsigned tag) {
         asm volatile(
-            "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, %5;\n\tsetp.ne.or.u32 p, %3, %5, p;\n\t"
-            "@p ld.relaxed.gpu.global.v4.b32 {%0, %1, %2, %3}, [%4];\n\t}"
-            : "+r"(v0), "+r"(t0), "+r"(v1), "+r"(t1)
-            : "l"(c), "r"(tag)
+            "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %3, %5;\n\tsetp.ne.or.u32 p, %4, %5, p;\n\t"
+            "@p ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];\n\t}"
+            : "+l"(w0), "+l"(w1)
+            : "l"(c), "r"(linkTag(w0)), "r"(linkTag(w1)), "r"(tag)
             : "memory");
     }
-    __device__ __forceinline__ bool ready(unsigned tag) const { return t0 == tag && t1 == tag; }
+    __device__ __forceinline__ bool ready(unsigned tag) const { return linkTag(w0) == tag && linkTag(w1) == tag; }
     __device__ __forceinline__ double value() const {
-        return __hiloint2double(static_cast<int>(v1), static_cast<int>(v0));
+        return __hiloint2double(static_cast<int>(static_cast<unsigned>(w1)), static_cast<int>(static_cast<unsigned>(w0)));
     }
 };
 template <>
 struct LinkReg<float> {
-    unsigned v0, t0;
-    __device__ __forceinline__ void set(unsigned tag) {
-        v0 = 0u;
-        t0 = tag;
-    }
+    unsigned long long w0;
+    __device__ __forceinline__ void set(unsigned tag) { w0 = linkWord(0u, tag); }
     __device__ __forceinline__ void load(const LinkCell<float>* c, unsigned tag) {
         asm volatile(
-            "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, %3;\n\t"
-            "@p ld.relaxed.gpu.global.v2.b32 {%0, %1}, [%2];\n\t}"
-            : "+r"(v0), "+r"(t0)
-            : "l"(c), "r"(tag)
+            "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, %3;\n\t"
+            "@p ld.relaxed.gpu.global.b64 %0, [%1];\n\t}"
+            : "+l"(w0)
+            : "l"(c), "r"(linkTag(w0)), "r"(tag)
             : "memory");
     }
-    __device__ __forceinline__ bool ready(unsigned tag) const { return t0 == tag; }
-    __device__ __forceinline__ float value() const { return __uint_as_float(v0); }
+    __device__ __forceinline__ bool ready(unsigned tag) const { return linkTag(w0) == tag; }
+    __device__ __forceinline__ float value() const { return __uint_as_float(static_cast<unsigned>(w0)); }
 };
 
 // The cells x[c[u]] of iteration `tag`, loaded until all of the warp's are
