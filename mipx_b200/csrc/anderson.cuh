@@ -54,8 +54,14 @@ struct AaArgs {
     const double* lb;  // scaled column bounds (clamp of the extrapolated x)
     const double* ub;
     int n, m, w, nb;
+    int prec;  // of the cycle graph these launches belong to
     double reg;
 };
+
+// A graph of the other precision than the state's: one queued before the host had
+// read that the iterates were handed over to FP64.  Nothing of it may run -- the
+// state still holds the restart that the cycle before it served.
+__device__ __forceinline__ bool aaStale(const AaArgs& a) { return a.st->prec != a.prec; }
 
 __device__ __forceinline__ bool aaRestartNow(const DevState* st) {
     return !st->done && st->restart && st->phase == 0;
@@ -78,7 +84,7 @@ __device__ __forceinline__ double aaBlockSum(double v) {
 
 template <class T>
 __global__ void __launch_bounds__(kBlock) aaStore(AaArgs a, const T* xh, const T* xi, const T* yh, const T* yi) {
-    if (!aaRestartNow(a.st) || a.st->prec != precTag<T>()) return;
+    if (aaStale(a) || !aaRestartNow(a.st)) return;
     const int n = a.n, dim = a.n + a.m, w = a.w;
     const int slot = a.as->count % w;
     const int filled = a.as->count < w ? a.as->count : w;  // slots holding a residual before this store
@@ -116,6 +122,7 @@ __global__ void __launch_bounds__(kBlock) aaStore(AaArgs a, const T* xh, const T
 // One warp: lanes reduce the partials of the new Gram row, lane 0 solves.
 __global__ void aaSolve(AaArgs a) {
     AaState* as = a.as;
+    if (aaStale(a)) return;
     if (!aaRestartNow(a.st)) {
         if (threadIdx.x == 0) {
             as->tried = 0;
@@ -185,7 +192,7 @@ __global__ void aaSolve(AaArgs a) {
 
 __global__ void __launch_bounds__(kBlock) aaExtrapolate(AaArgs a) {
     const AaState* as = a.as;
-    if (!as->tried) return;
+    if (aaStale(a) || !as->tried) return;
     const int dim = a.n + a.m, w = a.w, d = as->d;
     const double* alpha = a.work + 2 * w * w + w;
     const double* Rl = a.Rr + static_cast<size_t>(a.order[d - 1]) * dim;
@@ -213,7 +220,7 @@ __global__ void __launch_bounds__(kBlock) aaExtrapolate(AaArgs a) {
 
 __global__ void aaDecide(AaArgs a) {
     AaState* as = a.as;
-    if (threadIdx.x != 0 || !as->tried) return;
+    if (threadIdx.x != 0 || aaStale(a) || !as->tried) return;
     const int ldp = a.w > 2 ? a.w : 2;
     double s0 = 0.0, s1 = 0.0;
     for (int b = 0; b < a.nb; ++b) {
@@ -227,7 +234,7 @@ __global__ void aaDecide(AaArgs a) {
 // the anchor and the current iterate (pdlp.cpp:2437-2456).
 template <class T>
 __global__ void __launch_bounds__(kBlock) aaApply(AaArgs a, T* xi, T* yi, double* xc, double* yc, T* yg) {
-    if (!a.as->accepted || a.st->prec != precTag<T>()) return;
+    if (aaStale(a) || !a.as->accepted) return;
     const int n = a.n, m = a.m;
     const int total = n > m ? n : m;
     for (int k = blockIdx.x * kBlock + threadIdx.x; k < total; k += gridDim.x * kBlock) {

@@ -692,7 +692,7 @@ struct DeviceLp {
         a.N = o.termination_eval_frequency;
         return a;
     }
-    AaArgs aaArgs(double reg) const {
+    AaArgs aaArgs(double reg, int prec) const {
         AaArgs a{};
         a.X = aa_X;
         a.Rr = aa_R;
@@ -709,6 +709,7 @@ struct DeviceLp {
         a.m = m;
         a.w = aa_w;
         a.nb = aa_nb;
+        a.prec = prec;
         a.reg = reg;
         return a;
     }
@@ -1125,7 +1126,7 @@ int launchCycle(DeviceLp& d, const pdlpx_options& o, bool linked) {
     launches += launchChecks<T>(d, ca, s) - 2;
     controller<<<1, kBlock, 0, s>>>(d.st, d.dc, d.part_rows, d.part_cols, sizeof(T) == 8 ? 1 : 0);
     const int nb = std::max(1, std::min(gridFor(std::max(d.m, d.n), 1), 8 * d.sms));
-    const AaArgs aa = d.aaArgs(o.anderson_regularization);
+    const AaArgs aa = d.aaArgs(o.anderson_regularization, p);
     if (d.aa_w > 0) {
         aaStore<T><<<d.aa_nb, kBlock, 0, s>>>(aa, ia.xh, ia.xi, ia.yh, ia.yi);
         aaSolve<<<1, 32, 0, s>>>(aa);
