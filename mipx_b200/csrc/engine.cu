@@ -618,20 +618,39 @@ struct DeviceLp {
 
     // [FP32 / FP64][step launches / linked]
     cudaGraphExec_t cycle[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
-    int cycle_N[2][2] = {{0, 0}, {0, 0}};
     cudaGraphExec_t power = nullptr;
     int launches_cycle[2][2] = {{0, 0}, {0, 0}};
     int launches_power = 0;
     static constexpr int kPowerChunk = 8;  // even (powerChunkEnd)
 
+    // The options that the graphs above hold by value; a solve under other ones
+    // captures them anew.
+    struct GraphKey {
+        int N = 0, max_iter = 0, polish_max_iter = 0, sv_max_iter = 0;
+        double aa_reg = 0.0, sv_tol = 0.0;
+    } key;
+    void keepGraphsOf(const pdlpx_options& o) {
+        if (key.N != o.termination_eval_frequency || key.max_iter != o.max_iter ||
+            key.polish_max_iter != o.polish_max_iter || key.aa_reg != o.anderson_regularization) {
+            for (auto& row : cycle)
+                for (auto& g : row) drop(g);
+        }
+        if (key.sv_max_iter != o.sv_max_iter || key.sv_tol != o.sv_tol) drop(power);
+        key = GraphKey{o.termination_eval_frequency, o.max_iter, o.polish_max_iter, o.sv_max_iter,
+                       o.anderson_regularization, o.sv_tol};
+    }
+    static void drop(cudaGraphExec_t& g) {
+        if (g) cudaGraphExecDestroy(g);
+        g = nullptr;
+    }
+
     ~DeviceLp() {
         for (auto& row : cycle)
-            for (auto& g : row)
-                if (g) cudaGraphExecDestroy(g);
+            for (auto& g : row) drop(g);
         for (auto& row : kev)
             for (auto& e : row)
                 if (e) cudaEventDestroy(e);
-        if (power) cudaGraphExecDestroy(power);
+        drop(power);
         if (arena) cudaFree(arena);
         if (h_sb) cudaFreeHost(h_sb);
         for (auto& e : copied)
@@ -2228,6 +2247,7 @@ int32_t Engine::solveDevice(pdlpx_result* out) {
     }
     DeviceLp& d = *dev_;
     PDLPX_CK(cudaSetDevice(d.device));
+    d.keepGraphsOf(opt_);
     cudaStream_t s = d.stream;
     if (opt_.autotune && !d.tuned && d.nnz >= 100000) {
         const bool tp = opt_.spmv_group_at <= 0 && opt_.shape_primal <= 0;
@@ -2416,11 +2436,7 @@ int32_t Engine::solveDevice(pdlpx_result* out) {
     const LinkShare link_share(d.device, d.linked ? d.link_warps : 0);
     auto ensureCycle = [&](int prec, int link) -> int32_t {
         cudaGraphExec_t& exec = d.cycle[prec][link];
-        if (exec && d.cycle_N[prec][link] == N) return PDLPX_OK;
-        if (exec) {
-            cudaGraphExecDestroy(exec);
-            exec = nullptr;
-        }
+        if (exec) return PDLPX_OK;
         cudaGraph_t g = nullptr;
         PDLPX_CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
         d.launches_cycle[prec][link] =
@@ -2429,7 +2445,6 @@ int32_t Engine::solveDevice(pdlpx_result* out) {
         const cudaError_t ie = cudaGraphInstantiate(&exec, g, 0);
         cudaGraphDestroy(g);
         PDLPX_CK(ie);
-        d.cycle_N[prec][link] = N;
         return PDLPX_OK;
     };
 
