@@ -48,6 +48,7 @@
 #include <thread>
 #include <vector>
 
+#include "capture.hpp"
 #include "control.cuh"
 #include "engine.hpp"
 #include "kernels.cuh"
@@ -1207,9 +1208,15 @@ struct Pack {
         return e;
     }
 
+    auto linkedKernel() const { return link_lanes == 4 ? packLinked<4, 8> : packLinked<2, 4>; }
+    int linkedGrid(int sms) const {
+        const int units = static_cast<int>(h_pu.size() + h_du.size());
+        return std::min(sms, (units + link_warps - 1) / link_warps);
+    }
+
     // Whether the linked cycle runs the LPs with keep[l] set, and its unit lists,
     // uploaded on the pack's stream.
-    cudaError_t planLinked(const std::vector<char>& keep, int sms) {
+    cudaError_t planLinked(const std::vector<char>& keep, int device, int sms) {
         linked = false;
         link_warps = 0;
         if (!linkable) return cudaSuccess;
@@ -1233,7 +1240,11 @@ struct Pack {
         }
         const int64_t total_units = static_cast<int64_t>(h_pu.size() + h_du.size());
         link_warps = static_cast<int>(std::min<int64_t>(warps_max, (total_units + sms - 1) / sms));
-        linked = true;
+        linked = cooperativeFits(linkedKernel(), device, sms, linkedGrid(sms), 32 * link_warps);
+        if (!linked) {
+            link_warps = 0;
+            return cudaSuccess;
+        }
         cudaError_t e = cudaMemcpyAsync(d + o_pu, h_pu.data(), sizeof(int4) * h_pu.size(), cudaMemcpyHostToDevice, s);
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(d + o_du, h_du.data(), sizeof(int4) * h_du.size(), cudaMemcpyHostToDevice, s);
@@ -1241,7 +1252,7 @@ struct Pack {
     }
 
     // The steps of one cycle over the planned units.
-    int launchLinked(int N, int sms) {
+    int launchLinked(int N, int sms, cudaError_t& e) {
         LinkPackArgs q{P<int4>(o_pu),
                        P<int4>(o_du),
                        P<LinkLp>(o_lp),
@@ -1253,9 +1264,8 @@ struct Pack {
                        static_cast<int>(h_du.size()),
                        N};
         packLinkBegin<<<(L + 127) / 128, 128, 0, s>>>(args, q);
-        const int units = q.np + q.nd;
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(static_cast<unsigned>(std::min(sms, (units + link_warps - 1) / link_warps)));
+        cfg.gridDim = dim3(static_cast<unsigned>(linkedGrid(sms)));
         cfg.blockDim = dim3(static_cast<unsigned>(32 * link_warps));
         cfg.stream = s;
         cudaLaunchAttribute at[1];
@@ -1263,10 +1273,7 @@ struct Pack {
         at[0].val.cooperative = 1;
         cfg.attrs = at;
         cfg.numAttrs = 1;
-        if (link_lanes == 4)
-            cudaLaunchKernelEx(&cfg, packLinked<4, 8>, args, q);
-        else
-            cudaLaunchKernelEx(&cfg, packLinked<2, 4>, args, q);
+        e = cudaLaunchKernelEx(&cfg, linkedKernel(), args, q);
         return 2;
     }
 
@@ -1753,31 +1760,24 @@ int32_t solvePack(Pack& pk, const pdlpx_options& o, std::chrono::steady_clock::t
     int dev = 0, sms = 0;
     PDLPX_BCK(cudaGetDevice(&dev));
     PDLPX_BCK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    auto capture = [&](cudaGraphExec_t& g, int& count, bool power) -> int32_t {
-        if (g) {
-            cudaGraphExecDestroy(g);
-            g = nullptr;
-        }
-        cudaGraph_t graph = nullptr;
-        PDLPX_BCK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-        if (power)
-            count = pk.launchPower(kPowerChunk);
-        else if (&g == &pk.lcycle)
-            count = pk.launchLinked(o.termination_eval_frequency, sms) + pk.launchCycle(o.termination_eval_frequency, false);
-        else
-            count = pk.launchCycle(o.termination_eval_frequency, !pk.persist);
-        PDLPX_BCK(cudaStreamEndCapture(s, &graph));
-        const cudaError_t ie = cudaGraphInstantiate(&g, graph, 0);
-        cudaGraphDestroy(graph);
-        PDLPX_BCK(ie);
-        return PDLPX_OK;
+    auto capture = [&](cudaGraphExec_t& g, int& count, bool power) -> cudaError_t {
+        return captureGraph(s, g, [&] {
+            cudaError_t e = cudaSuccess;
+            if (power)
+                count = pk.launchPower(kPowerChunk);
+            else if (&g == &pk.lcycle)
+                count = pk.launchLinked(o.termination_eval_frequency, sms, e) +
+                        pk.launchCycle(o.termination_eval_frequency, false);
+            else
+                count = pk.launchCycle(o.termination_eval_frequency, !pk.persist);
+            return e;
+        });
     };
     auto stopped = [&]() { return stop != nullptr && stop->load(std::memory_order_relaxed) != 0; };
 
     // ---- power iteration of every LP
     if (o.sv_max_iter > 0) {
-        int32_t rc = capture(pk.power, pk.power_launches, true);
-        if (rc != PDLPX_OK) return rc;
+        PDLPX_BCK(capture(pk.power, pk.power_launches, true));
         for (int guard = 0; guard < 2 + o.sv_max_iter / kPowerChunk; ++guard) {
             PDLPX_BCK(cudaGraphLaunch(pk.power, s));
             launches += pk.power_launches;
@@ -1868,7 +1868,7 @@ int32_t solvePack(Pack& pk, const pdlpx_options& o, std::chrono::steady_clock::t
 
     // ---- restart cycles; finished LPs are read back after the cycle that ends them
     std::vector<char> keep(L, 1), collected(L, 0);
-    if (!pk.persist) PDLPX_BCK(pk.planLinked(keep, sms));
+    if (!pk.persist) PDLPX_BCK(pk.planLinked(keep, dev, sms));
     LinkShare share(dev, pk.link_warps);
     int perr = 0;
     SleepWait sleeper;
@@ -1880,13 +1880,14 @@ int32_t solvePack(Pack& pk, const pdlpx_options& o, std::chrono::steady_clock::t
             PDLPX_BCK(pk.launchPersistent(o.termination_eval_frequency));
             ++launches;
         }
-        const bool linked = pk.linked && share.fits();
-        cudaGraphExec_t& graph = linked ? pk.lcycle : pk.cycle;
-        int& graph_launches = linked ? pk.lcycle_launches : pk.cycle_launches;
-        if (!graph) {
-            const int32_t rc = capture(graph, graph_launches, false);
-            if (rc != PDLPX_OK) return rc;
+        bool linked = pk.linked && share.fits();
+        if (linked && !pk.lcycle && capture(pk.lcycle, pk.lcycle_launches, false) != cudaSuccess) {
+            pk.linkable = pk.linked = linked = false;  // the same bits by launches
+            share.set(0);
         }
+        cudaGraphExec_t& graph = linked ? pk.lcycle : pk.cycle;
+        const int& graph_launches = linked ? pk.lcycle_launches : pk.cycle_launches;
+        if (!graph) PDLPX_BCK(capture(pk.cycle, pk.cycle_launches, false));
         PDLPX_BCK(cudaGraphLaunch(graph, s));
         launches += graph_launches;
         ++cycles;
@@ -1941,7 +1942,7 @@ int32_t solvePack(Pack& pk, const pdlpx_options& o, std::chrono::steady_clock::t
             if (pk.persist)
                 PDLPX_BCK(pk.uploadPersistTiles());
             else
-                PDLPX_BCK(pk.planLinked(keep, sms));
+                PDLPX_BCK(pk.planLinked(keep, dev, sms));
             share.set(pk.link_warps);
             for (cudaGraphExec_t* g : {&pk.cycle, &pk.lcycle}) {
                 if (*g) cudaGraphExecDestroy(*g);

@@ -22,6 +22,7 @@
 #include <random>
 
 #include "engine.hpp"
+#include "capture.hpp"
 #include "kernels.cuh"
 #include "anderson.cuh"
 #include "control.cuh"
@@ -612,6 +613,7 @@ struct DeviceLp {
     bool linked = false;
     int link_lanes = 4;
     int link_warps = 0;  // of its grid per SM
+    bool link_refused = false;  // its launch failed on this image: the step launches run
     int tiny = 0;        // one block runs it (tiny.cuh): 1 short columns, 2 short rows
     int sell_max[2] = {0, 0};  // most entries of a sliced-ELL column / row
     void *link_x = nullptr, *link_y = nullptr;  // cells (null: the launches run)
@@ -1031,10 +1033,27 @@ bool linkable(const DeviceLp& d, const pdlpx_options& o) {
     if (d.longest > 1000) return false;
     return d.nnz <= (csr ? 90000 : (d.nlP > 0 || d.nlD > 0) ? 350000 : 600000);
 }
+// f(kernel, lanes per sliced-ELL column, lanes per sliced-ELL row) of the planned grid.
+template <class T, class F>
+auto withLinked(const DeviceLp& d, F f) {
+    if (linkCsr(d)) return d.link_lanes == 1 ? f(linkedSteps<1, 8, true, T>, 1, 8) : f(linkedSteps<4, 8, true, T>, 4, 8);
+    switch (d.link_lanes) {
+        case 1: return f(linkedSteps<1, 8, false, T>, 1, 8);
+        case 2: return f(linkedSteps<2, 4, false, T>, 2, 4);
+        case 4: return f(linkedSteps<4, 8, false, T>, 4, 8);
+        default: return f(linkedSteps<8, 4, false, T>, 8, 4);
+    }
+}
+int linkedUnits(const DeviceLp& d, bool primal, int sub) {
+    const int shape = primal ? d.shapeP : d.shapeD;
+    return linkUnits(primal ? d.n : d.m, primal ? d.nlP : d.nlD, isSell(shape) ? 0 : kShapes[shape].G, sub);
+}
+int linkedGrid(const DeviceLp& d, int units) { return std::min(d.sms, (units + d.link_warps - 1) / d.link_warps); }
+
 void planLinked(DeviceLp& d) {
     // rowDotU with two sums per lane (the autotuner may pick it) has no linked form
     auto supported = [](int shape) { return isSell(shape) || kShapes[shape].U >= kLinkU; };
-    d.linked = d.link_x != nullptr && supported(d.shapeP) && supported(d.shapeD);
+    d.linked = d.link_x != nullptr && !d.link_refused && supported(d.shapeP) && supported(d.shapeD);
     d.tiny = d.link_warps = 0;
     if (!d.linked) return;
     if (!linkCsr(d) && (d.n + kSlice - 1) / kSlice + (d.m + kSlice - 1) / kSlice <= kTinyWarps) {
@@ -1046,33 +1065,18 @@ void planLinked(DeviceLp& d) {
     if (d.tiny != 0) return;
     const double mean = static_cast<double>(d.nnz - d.zlP) / std::max(1, d.n - d.nlP);
     d.link_lanes = mean <= 3.0 ? 1 : mean > 14.0 ? 8 : d.nnz <= 240000 ? 4 : 2;
-    const bool csr = linkCsr(d);
-    const int lanes_p = csr && d.link_lanes != 1 ? 4 : d.link_lanes;
-    const int lanes_d = csr || d.link_lanes == 1 || d.link_lanes == 4 ? 8 : 4;
     // one warp per unit over all SMs first (a unit's gathers queue in its SM's
     // L1), and no wider blocks than that takes: small LPs leave room for the
     // grids of other solvers
-    const int units = linkUnits(d.n, d.nlP, isSell(d.shapeP) ? 0 : kShapes[d.shapeP].G, lanes_p) +
-                      linkUnits(d.m, d.nlD, isSell(d.shapeD) ? 0 : kShapes[d.shapeD].G, lanes_d);
-    d.link_warps = std::min(linkThreads(csr) / 32, (units + d.sms - 1) / d.sms);
+    auto plan = [&](auto kernel, int lp, int ld) {
+        const int units = linkedUnits(d, true, lp) + linkedUnits(d, false, ld);
+        d.link_warps = std::min(linkThreads(linkCsr(d)) / 32, (units + d.sms - 1) / d.sms);
+        return cooperativeFits(kernel, d.device, d.sms, linkedGrid(d, units), 32 * d.link_warps);
+    };
+    d.linked = withLinked<double>(d, plan) && (!d.mixed || withLinked<float>(d, plan));
+    if (!d.linked) d.link_warps = 0;
 }
 
-template <int LP, int LD, bool CSR, class T>
-cudaError_t launchLinkedAs(const DeviceLp& d, LinkArgs<T>& a, cudaStream_t s) {
-    a.P.units = linkUnits(a.P.rows, a.P.nl, a.P.lanes, LP);
-    a.D.units = linkUnits(a.D.rows, a.D.nl, a.D.lanes, LD);
-    const int units = a.P.units + a.D.units;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(static_cast<unsigned>(std::min(d.sms, (units + d.link_warps - 1) / d.link_warps)));
-    cfg.blockDim = dim3(static_cast<unsigned>(32 * d.link_warps));
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, linkedSteps<LP, LD, CSR, T>, a);
-}
 template <class T>
 cudaError_t launchLinked(const DeviceLp& d, const IterArgs<T>& ia, cudaStream_t s) {
     LinkArgs<T> a{};
@@ -1091,14 +1095,20 @@ cudaError_t launchLinked(const DeviceLp& d, const IterArgs<T>& ia, cudaStream_t 
             tinySteps<kTinyLong, kTinyShort, T><<<1, threads, 0, s>>>(a);
         return cudaGetLastError();
     }
-    if (linkCsr(d))
-        return d.link_lanes == 1 ? launchLinkedAs<1, 8, true, T>(d, a, s) : launchLinkedAs<4, 8, true, T>(d, a, s);
-    switch (d.link_lanes) {
-        case 1: return launchLinkedAs<1, 8, false, T>(d, a, s);
-        case 2: return launchLinkedAs<2, 4, false, T>(d, a, s);
-        case 4: return launchLinkedAs<4, 8, false, T>(d, a, s);
-        default: return launchLinkedAs<8, 4, false, T>(d, a, s);
-    }
+    return withLinked<T>(d, [&](auto kernel, int lp, int ld) {
+        a.P.units = linkedUnits(d, true, lp);
+        a.D.units = linkedUnits(d, false, ld);
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(static_cast<unsigned>(linkedGrid(d, a.P.units + a.D.units)));
+        cfg.blockDim = dim3(static_cast<unsigned>(32 * d.link_warps));
+        cfg.stream = s;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeCooperative;
+        at[0].val.cooperative = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        return cudaLaunchKernelEx(&cfg, kernel, a);
+    });
 }
 
 // FP64 check pass: short rows write partials [0, nb_*_s), long rows the rest.
@@ -1120,7 +1130,7 @@ int launchChecks(const DeviceLp& d, const CheckArgs<T>& ca, cudaStream_t s) {
 
 // One restart cycle: N fused iterations, check, controller, restart copy.
 template <class T>
-int launchCycle(DeviceLp& d, const pdlpx_options& o, bool linked) {
+int launchCycle(DeviceLp& d, const pdlpx_options& o, bool linked, cudaError_t& e) {
     const IterArgs<T> ia = iterArgs<T>(d, o);
     const CheckArgs<T> ca = d.check<T>(ia.xh, ia.xi, ia.yh, ia.yi);
     cudaStream_t s = d.stream;
@@ -1130,8 +1140,9 @@ int launchCycle(DeviceLp& d, const pdlpx_options& o, bool linked) {
     // becomes an event-record node of the graph (a plain record would only
     // mark a dependency), so every replay records it on the device.
     auto mark = [&](cudaEvent_t e) { cudaEventRecordWithFlags(e, s, cudaEventRecordExternal); };
+    e = cudaSuccess;
     if (linked) {
-        launchLinked<T>(d, ia, s);
+        e = launchLinked<T>(d, ia, s);
         ++launches;
     }
     for (int k = 1; !linked && k <= o.termination_eval_frequency; ++k) {
@@ -2293,19 +2304,16 @@ int32_t Engine::solveDevice(pdlpx_result* out) {
         pa.tol = opt_.sv_tol;
         if (!d.power) {
             // FP32 matrix values in mixed mode, FP64 in FP64 mode; vectors and sums FP64.
-            cudaGraph_t g = nullptr;
-            PDLPX_CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-            if (d.mixed) {
-                const PowerMat<float> mt{d.a_ptr, d.a_idx, d.a_v32, d.at_ptr, d.at_idx, d.at_v32};
-                d.launches_power = launchPowerChunk(d, pa, mt, DeviceLp::kPowerChunk);
-            } else {
-                const PowerMat<double> mt{d.a_ptr, d.a_idx, d.a_v64, d.at_ptr, d.at_idx, d.at_v64};
-                d.launches_power = launchPowerChunk(d, pa, mt, DeviceLp::kPowerChunk);
-            }
-            PDLPX_CK(cudaStreamEndCapture(s, &g));
-            const cudaError_t ie = cudaGraphInstantiate(&d.power, g, 0);
-            cudaGraphDestroy(g);
-            PDLPX_CK(ie);
+            PDLPX_CK(captureGraph(s, d.power, [&] {
+                if (d.mixed) {
+                    const PowerMat<float> mt{d.a_ptr, d.a_idx, d.a_v32, d.at_ptr, d.at_idx, d.at_v32};
+                    d.launches_power = launchPowerChunk(d, pa, mt, DeviceLp::kPowerChunk);
+                } else {
+                    const PowerMat<double> mt{d.a_ptr, d.a_idx, d.a_v64, d.at_ptr, d.at_idx, d.at_v64};
+                    d.launches_power = launchPowerChunk(d, pa, mt, DeviceLp::kPowerChunk);
+                }
+                return cudaSuccess;
+            }));
         }
         for (int guard = 0; guard < 1 + opt_.sv_max_iter / DeviceLp::kPowerChunk + 1; ++guard) {
             if (d.h_ps->done) break;
@@ -2433,19 +2441,15 @@ int32_t Engine::solveDevice(pdlpx_result* out) {
         PDLPX_CK(cudaMemsetAsync(d.link_y, 0, sizeof(LinkCell<double>) * static_cast<size_t>(m), s));
     }
     // ---- capture the restart-cycle graphs lazily
-    const LinkShare link_share(d.device, d.linked ? d.link_warps : 0);
-    auto ensureCycle = [&](int prec, int link) -> int32_t {
-        cudaGraphExec_t& exec = d.cycle[prec][link];
-        if (exec) return PDLPX_OK;
-        cudaGraph_t g = nullptr;
-        PDLPX_CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-        d.launches_cycle[prec][link] =
-            prec == 0 ? launchCycle<float>(d, opt_, link != 0) : launchCycle<double>(d, opt_, link != 0);
-        PDLPX_CK(cudaStreamEndCapture(s, &g));
-        const cudaError_t ie = cudaGraphInstantiate(&exec, g, 0);
-        cudaGraphDestroy(g);
-        PDLPX_CK(ie);
-        return PDLPX_OK;
+    LinkShare link_share(d.device, d.linked ? d.link_warps : 0);
+    auto ensureCycle = [&](int prec, int link) -> cudaError_t {
+        if (d.cycle[prec][link]) return cudaSuccess;
+        return captureGraph(s, d.cycle[prec][link], [&] {
+            cudaError_t e = cudaSuccess;
+            d.launches_cycle[prec][link] =
+                prec == 0 ? launchCycle<float>(d, opt_, link != 0, e) : launchCycle<double>(d, opt_, link != 0, e);
+            return e;
+        });
     };
 
     used_gpu_ = true;
@@ -2473,8 +2477,15 @@ int32_t Engine::solveDevice(pdlpx_result* out) {
         ~Drain() { cudaStreamSynchronize(s); }
     } drain{s};
     auto enqueue = [&](int link) -> int32_t {
-        const int32_t rc = ensureCycle(prec, link);
-        if (rc != PDLPX_OK) return rc;
+        cudaError_t e = ensureCycle(prec, link);
+        if (e != cudaSuccess && link) {  // the same bits by launches
+            d.link_refused = true;
+            d.linked = false;
+            link_share.set(0);
+            link = 0;
+            e = ensureCycle(prec, link);
+        }
+        PDLPX_CK(e);
         const int slot = (head + queued) & 1;
         PDLPX_CK(cudaGraphLaunch(d.cycle[prec][link], s));
         launches += d.launches_cycle[prec][link];

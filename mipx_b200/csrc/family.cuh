@@ -1194,58 +1194,49 @@ int32_t solveFamilyPack(FamPack& fp, const pdlpx_options& o, std::chrono::steady
     auto hostSeconds = [&]() { return std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count(); };
     auto stopped = [&]() { return stop != nullptr && stop->load(std::memory_order_relaxed) != 0; };
     std::vector<int> h_flags(kFam);
-    auto capture = [&](cudaGraphExec_t& gx, int& count, bool power) -> int32_t {
-        if (gx) {
-            cudaGraphExecDestroy(gx);
-            gx = nullptr;
-        }
+    auto capture = [&](cudaGraphExec_t& gx, int& count, bool power) -> cudaError_t {
         const FamArgs args = fp.args;
         const int stepRows = args.gb + args.gk;
         const int ctl = (args.L + kCtlWarps - 1) / kCtlWarps;
         const int nrs = std::max(1, std::min<int>(static_cast<int>((fp.colsAll() + fp.rowsAll() + kBlock - 1) / kBlock),
                                                   8 * sms));
-        cudaGraph_t graph = nullptr;
-        PDLPX_BCK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-        count = 0;
-        if (power) {
-            for (int r = 0; r < 8; ++r) {
-                famPowerA<<<stepRows, kBlock, 0, s>>>(args);
-                famPowerAt<<<args.nbc, kBlock, 0, s>>>(args);
-                famPowerFinish1<<<ctl, 32 * kCtlWarps, 0, s>>>(args);
-                famPowerNormalize<<<args.nbc, kBlock, 0, s>>>(args);
-                famPowerFinish2<<<ctl, 32 * kCtlWarps, 0, s>>>(args);
+        return captureGraph(s, gx, [&] {
+            count = 0;
+            if (power) {
+                for (int r = 0; r < 8; ++r) {
+                    famPowerA<<<stepRows, kBlock, 0, s>>>(args);
+                    famPowerAt<<<args.nbc, kBlock, 0, s>>>(args);
+                    famPowerFinish1<<<ctl, 32 * kCtlWarps, 0, s>>>(args);
+                    famPowerNormalize<<<args.nbc, kBlock, 0, s>>>(args);
+                    famPowerFinish2<<<ctl, 32 * kCtlWarps, 0, s>>>(args);
+                    count += 5;
+                }
+            } else {
+                for (int k = 1; k <= o.termination_eval_frequency; ++k) {
+                    auto primal = args.cpw == 1 ? (args.listed ? famPrimal<1, true> : famPrimal<1, false>)
+                                                : (args.listed ? famPrimal<kFamColsPerWarp, true>
+                                                               : famPrimal<kFamColsPerWarp, false>);
+                    primal<<<args.gp, kBlock, 0, s>>>(args, k);
+                    if (args.rpw == 1)
+                        famDual<1><<<args.gd + args.gk, kBlock, 0, s>>>(args, k);
+                    else
+                        famDual<kFamRowsPerWarp><<<args.gd + args.gk, kBlock, 0, s>>>(args, k);
+                    count += 2;
+                }
+                famCheckRows<<<args.nbr + args.nbk, kBlock, 0, s>>>(args);
+                famCheckCols<<<args.nbc, kBlock, 0, s>>>(args);
+                famController<<<ctl, 32 * kCtlWarps, 0, s>>>(args);
+                famRestart<<<nrs, kBlock, 0, s>>>(args);
+                famFinish<<<1, kFam, 0, s>>>(args);
                 count += 5;
             }
-        } else {
-            for (int k = 1; k <= o.termination_eval_frequency; ++k) {
-                auto primal = args.cpw == 1 ? (args.listed ? famPrimal<1, true> : famPrimal<1, false>)
-                                            : (args.listed ? famPrimal<kFamColsPerWarp, true>
-                                                           : famPrimal<kFamColsPerWarp, false>);
-                primal<<<args.gp, kBlock, 0, s>>>(args, k);
-                if (args.rpw == 1)
-                    famDual<1><<<args.gd + args.gk, kBlock, 0, s>>>(args, k);
-                else
-                    famDual<kFamRowsPerWarp><<<args.gd + args.gk, kBlock, 0, s>>>(args, k);
-                count += 2;
-            }
-            famCheckRows<<<args.nbr + args.nbk, kBlock, 0, s>>>(args);
-            famCheckCols<<<args.nbc, kBlock, 0, s>>>(args);
-            famController<<<ctl, 32 * kCtlWarps, 0, s>>>(args);
-            famRestart<<<nrs, kBlock, 0, s>>>(args);
-            famFinish<<<1, kFam, 0, s>>>(args);
-            count += 5;
-        }
-        PDLPX_BCK(cudaStreamEndCapture(s, &graph));
-        const cudaError_t ie = cudaGraphInstantiate(&gx, graph, 0);
-        cudaGraphDestroy(graph);
-        PDLPX_BCK(ie);
-        return PDLPX_OK;
+            return cudaSuccess;
+        });
     };
     // power iteration of every lane whose PowerState is not done, then the step sizes
     auto powerPhase = [&]() -> int32_t {
         if (o.sv_max_iter > 0) {
-            int32_t rc = capture(fp.power, fp.power_launches, true);
-            if (rc != PDLPX_OK) return rc;
+            PDLPX_BCK(capture(fp.power, fp.power_launches, true));
             for (int guard = 0; guard < 2 + o.sv_max_iter / 8; ++guard) {
                 PDLPX_BCK(cudaGraphLaunch(fp.power, s));
                 launches += fp.power_launches;
@@ -1265,8 +1256,7 @@ int32_t solveFamilyPack(FamPack& fp, const pdlpx_options& o, std::chrono::steady
     {
         int32_t rc = powerPhase();
         if (rc != PDLPX_OK) return rc;
-        rc = capture(fp.cycle, fp.cycle_launches, false);
-        if (rc != PDLPX_OK) return rc;
+        PDLPX_BCK(capture(fp.cycle, fp.cycle_launches, false));
     }
 
     // ---- admission: members that arrive while the pack runs take free lanes
@@ -1405,7 +1395,8 @@ int32_t solveFamilyPack(FamPack& fp, const pdlpx_options& o, std::chrono::steady
         setShape(fp.args);
         int32_t rc = powerPhase();
         if (rc != PDLPX_OK) return rc;
-        return capture(fp.cycle, fp.cycle_launches, false);
+        PDLPX_BCK(capture(fp.cycle, fp.cycle_launches, false));
+        return PDLPX_OK;
     };
 
     // ---- restart cycles
