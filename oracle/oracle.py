@@ -28,6 +28,10 @@ REF_BOUND_LIB = HERE / "_ref" / "libmipx_pdlp_bound.so"
 _libs: dict = {}
 
 
+class ReferenceNotBuilt(FileNotFoundError):
+    """A library compiled from the reference's sources, on a machine that never had them."""
+
+
 def reference_dir() -> Path | None:
     """The mipx source tree the reference libraries are compiled from:
     $MIPX_REFERENCE_DIR, else the checkout the oracle's Makefile recipe reads
@@ -55,7 +59,7 @@ def _load(path: Path):
             if path == ORACLE_LIB:
                 build(ref=False)
             else:
-                raise FileNotFoundError(f"{path} not built (reference sources needed at build time)")
+                raise ReferenceNotBuilt(f"{path} not built (reference sources needed at build time)")
         from mipx_b200 import _capi  # struct layouts only
         lib = C.CDLL(str(path))
         sig = [C.POINTER(_capi.Lp), C.POINTER(_capi.Options), C.POINTER(_capi.Result), _capi.P_f64, _capi.P_f64]
