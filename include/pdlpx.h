@@ -171,7 +171,10 @@ typedef struct pdlpx_options {
                                          window, the whole side.  A window keeps each row within that many
                                          places of its original position (for LPs whose numbering gives
                                          the gathers locality) */
-    int32_t reserved[1];
+    int32_t link_polls;               /* loads after which a warp of the linked restart cycle gives up
+                                         waiting for a value (the solve then returns
+                                         PDLPX_E_TIMEOUT; the solver stays usable): <= 0 (default)
+                                         4,194,304, about two seconds */
 } pdlpx_options;
 
 /* Image of mipx::LpResult (lp_solver.h:11-16) plus engine diagnostics. */

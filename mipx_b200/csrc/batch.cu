@@ -325,7 +325,7 @@ struct LinkPackArgs {
     LinkCell<float>* xf;
     LinkCell<double>* xd;
     LinkCell<double>* y;
-    int* err;
+    LinkWait wait;
     int np, nd, N;
 };
 constexpr int kLinkPackThreads = 512;
@@ -354,7 +354,7 @@ __global__ void packLinkBegin(PackArgs a, LinkPackArgs q) {
 template <int L, class T>
 __device__ __forceinline__ void linkPackPrimal(const IterArgs<T>& p, const int* idx, const T* val, int2 h, int r,
                                                int lane, int j, const LinkLp& lp, int it, double lam,
-                                               const LinkCell<double>* y, LinkCell<T>* x, int* err, bool& ok) {
+                                               const LinkCell<double>* y, LinkCell<T>* x, const LinkWait& wait, bool& ok) {
     ColPack<T> c{};
     double xcd = 0.0, xi = 0.0, tau = 0.0;
     if (j >= 0) {
@@ -364,7 +364,7 @@ __device__ __forceinline__ void linkPackPrimal(const IterArgs<T>& p, const int* 
         tau = lp.step * static_cast<double>(c.tau) / lp.pw;
     }
     const unsigned tag = lp.base + static_cast<unsigned>(it);
-    const double s = linkSellDot<L>(idx, val, h, r, lane, y, tag - 1u, err, ok);
+    const double s = linkSellDot<L>(idx, val, h, r, lane, y, tag - 1u, wait, ok);
     if (j < 0) return;
     double xh, xr;
     const double xn = primalValues<T>(c, xcd, xi, s, tau, lam, xh, xr);
@@ -375,7 +375,7 @@ __device__ __forceinline__ void linkPackPrimal(const IterArgs<T>& p, const int* 
 template <int L, class T>
 __device__ __forceinline__ void linkPackDual(const IterArgs<T>& p, const int* idx, const T* val, int2 h, int r,
                                              int lane, int i, const LinkLp& lp, int it, double lam,
-                                             const LinkCell<T>* x, LinkCell<double>* y, int* err, bool& ok) {
+                                             const LinkCell<T>* x, LinkCell<double>* y, const LinkWait& wait, bool& ok) {
     RowPack<T> c{};
     double ycd = 0.0, yi = 0.0;
     if (i >= 0) {
@@ -384,7 +384,7 @@ __device__ __forceinline__ void linkPackDual(const IterArgs<T>& p, const int* id
         yi = static_cast<double>(p.yi[i]);
     }
     const unsigned tag = lp.base + static_cast<unsigned>(it);
-    const double s = linkSellDot<L>(idx, val, h, r, lane, x, tag, err, ok);
+    const double s = linkSellDot<L>(idx, val, h, r, lane, x, tag, wait, ok);
     if (i < 0) return;
     double py;
     const double yn = dualValues<T>(c, ycd, yi, s, lp.step, lp.pw, lam, py);
@@ -396,6 +396,7 @@ __device__ __forceinline__ void linkPackDual(const IterArgs<T>& p, const int* id
 // LP / LD: lanes per column / row.
 template <int LP, int LD>
 __global__ void __launch_bounds__(kLinkPackThreads, 1) packLinked(PackArgs a, LinkPackArgs q) {
+    if (linkFailed(q.wait)) return;
     const int lane = static_cast<int>(threadIdx.x) & 31;
     const int wid = static_cast<int>(blockIdx.x) + static_cast<int>(gridDim.x) * (static_cast<int>(threadIdx.x) >> 5);
     const int nw = static_cast<int>(gridDim.x) * (static_cast<int>(blockDim.x) >> 5);
@@ -422,9 +423,9 @@ __global__ void __launch_bounds__(kLinkPackThreads, 1) packLinked(PackArgs a, Li
             const int j = rowOf(d, LP), r = (d.y & 31) + lane / LP;
             const int2 h = __ldg(a.cs.hdr + d.w);
             if (lp.prec == 0)
-                linkPackPrimal<LP, float>(a.it32, a.cs.idx, a.cs.v32, h, r, lane, j, lp, it, lam, q.y, q.xf, q.err, ok);
+                linkPackPrimal<LP, float>(a.it32, a.cs.idx, a.cs.v32, h, r, lane, j, lp, it, lam, q.y, q.xf, q.wait, ok);
             else
-                linkPackPrimal<LP, double>(a.it64, a.cs.idx, a.cs.v64, h, r, lane, j, lp, it, lam, q.y, q.xd, q.err, ok);
+                linkPackPrimal<LP, double>(a.it64, a.cs.idx, a.cs.v64, h, r, lane, j, lp, it, lam, q.y, q.xd, q.wait, ok);
         }
         __syncwarp();
         for (int u = firstD; u < q.nd; u += nw) {
@@ -436,9 +437,9 @@ __global__ void __launch_bounds__(kLinkPackThreads, 1) packLinked(PackArgs a, Li
             const int i = rowOf(d, LD), r = (d.y & 31) + lane / LD;
             const int2 h = __ldg(a.rs.hdr + d.w);
             if (lp.prec == 0)
-                linkPackDual<LD, float>(a.it32, a.rs.idx, a.rs.v32, h, r, lane, i, lp, it, lam, q.xf, q.y, q.err, ok);
+                linkPackDual<LD, float>(a.it32, a.rs.idx, a.rs.v32, h, r, lane, i, lp, it, lam, q.xf, q.y, q.wait, ok);
             else
-                linkPackDual<LD, double>(a.it64, a.rs.idx, a.rs.v64, h, r, lane, i, lp, it, lam, q.xd, q.y, q.err, ok);
+                linkPackDual<LD, double>(a.it64, a.rs.idx, a.rs.v64, h, r, lane, i, lp, it, lam, q.xd, q.y, q.wait, ok);
         }
         __syncwarp();
         if (__any_sync(0xffffffffu, !ok)) return;
@@ -1252,14 +1253,14 @@ struct Pack {
     }
 
     // The steps of one cycle over the planned units.
-    int launchLinked(int N, int sms, cudaError_t& e) {
+    int launchLinked(int N, int polls, int sms, cudaError_t& e) {
         LinkPackArgs q{P<int4>(o_pu),
                        P<int4>(o_du),
                        P<LinkLp>(o_lp),
                        mixed ? P<LinkCell<float>>(o_lxf) : nullptr,
                        P<LinkCell<double>>(o_lxd),
                        P<LinkCell<double>>(o_ly),
-                       P<int>(o_flags) + L,
+                       LinkWait{P<int>(o_flags) + L, polls},
                        static_cast<int>(h_pu.size()),
                        static_cast<int>(h_du.size()),
                        N};
@@ -1766,7 +1767,7 @@ int32_t solvePack(Pack& pk, const pdlpx_options& o, std::chrono::steady_clock::t
             if (power)
                 count = pk.launchPower(kPowerChunk);
             else if (&g == &pk.lcycle)
-                count = pk.launchLinked(o.termination_eval_frequency, sms, e) +
+                count = pk.launchLinked(o.termination_eval_frequency, linkPolls(o.link_polls), sms, e) +
                         pk.launchCycle(o.termination_eval_frequency, false);
             else
                 count = pk.launchCycle(o.termination_eval_frequency, !pk.persist);

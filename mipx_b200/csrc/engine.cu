@@ -628,17 +628,17 @@ struct DeviceLp {
     // The options that the graphs above hold by value; a solve under other ones
     // captures them anew.
     struct GraphKey {
-        int N = 0, max_iter = 0, polish_max_iter = 0, sv_max_iter = 0;
+        int N = 0, max_iter = 0, polish_max_iter = 0, link_polls = 0, sv_max_iter = 0;
         double aa_reg = 0.0, sv_tol = 0.0;
     } key;
     void keepGraphsOf(const pdlpx_options& o) {
         if (key.N != o.termination_eval_frequency || key.max_iter != o.max_iter ||
-            key.polish_max_iter != o.polish_max_iter || key.aa_reg != o.anderson_regularization) {
+            key.polish_max_iter != o.polish_max_iter || key.link_polls != o.link_polls || key.aa_reg != o.anderson_regularization) {
             for (auto& row : cycle)
                 for (auto& g : row) drop(g);
         }
         if (key.sv_max_iter != o.sv_max_iter || key.sv_tol != o.sv_tol) drop(power);
-        key = GraphKey{o.termination_eval_frequency, o.max_iter, o.polish_max_iter, o.sv_max_iter,
+        key = GraphKey{o.termination_eval_frequency, o.max_iter, o.polish_max_iter, o.link_polls, o.sv_max_iter,
                        o.anderson_regularization, o.sv_tol};
     }
     static void drop(cudaGraphExec_t& g) {
@@ -1078,14 +1078,14 @@ void planLinked(DeviceLp& d) {
 }
 
 template <class T>
-cudaError_t launchLinked(const DeviceLp& d, const IterArgs<T>& ia, cudaStream_t s) {
+cudaError_t launchLinked(const DeviceLp& d, const IterArgs<T>& ia, int polls, cudaStream_t s) {
     LinkArgs<T> a{};
     a.it = ia;
     a.P = linkSide<T>(d, ia, true);
     a.D = linkSide<T>(d, ia, false);
     a.x = static_cast<LinkCell<T>*>(d.link_x);
     a.y = static_cast<LinkCell<T>*>(d.link_y);
-    a.err = &reinterpret_cast<StateBlock*>(d.st)->link_err;
+    a.wait = LinkWait{&reinterpret_cast<StateBlock*>(d.st)->link_err, linkPolls(polls)};
     a.time = &reinterpret_cast<StateBlock*>(d.st)->lt;
     if (d.tiny != 0) {
         const int threads = 32 * ((d.n + kSlice - 1) / kSlice + (d.m + kSlice - 1) / kSlice);
@@ -1142,7 +1142,7 @@ int launchCycle(DeviceLp& d, const pdlpx_options& o, bool linked, cudaError_t& e
     auto mark = [&](cudaEvent_t e) { cudaEventRecordWithFlags(e, s, cudaEventRecordExternal); };
     e = cudaSuccess;
     if (linked) {
-        e = launchLinked<T>(d, ia, s);
+        e = launchLinked<T>(d, ia, o.link_polls, s);
         ++launches;
     }
     for (int k = 1; !linked && k <= o.termination_eval_frequency; ++k) {

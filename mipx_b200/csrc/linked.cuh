@@ -28,7 +28,8 @@
 // Why it always ends: a warp runs its columns' step k, then its rows' step k,
 // and waits only for cells of strictly earlier half-steps; every block is
 // resident (cooperative launch).  Should a block be kept from running all the
-// same, waits end after kLinkPolls loads, set the error word and leave.
+// same, waits end after LinkWait::polls loads, set the error word and leave, and
+// a launch that finds it set does nothing.
 //
 // Every row is summed in the order of the per-step kernels (sellDot, rowDotU +
 // groupSum) and updated by the same expressions: iterates are the same bits.
@@ -42,6 +43,14 @@
 namespace pdlpx {
 
 constexpr int kLinkPolls = 1 << 22;  // ~2 s of L2 round trips
+inline int linkPolls(int option) { return option > 0 ? option : kLinkPolls; }
+
+// How the waits of a launch end when what they wait for does not come.
+struct LinkWait {
+    int* err;   // error word, set by the first wait that runs out
+    int polls;  // loads of a cell until then
+};
+__device__ __forceinline__ bool linkFailed(const LinkWait& w) { return *reinterpret_cast<volatile int*>(w.err) != 0; }
 
 constexpr int kLinkU = 4;  // cells per lane per round
 // Sleep between polls (ns) beside CSR rows: their LPs have few rows or columns that
@@ -163,7 +172,7 @@ struct LinkReg<float> {
 // ran out.
 template <int U, int NAP, class V, class X>
 __device__ __forceinline__ bool linkGather(const LinkCell<X>* __restrict__ x, const int (&c)[U], const V (&v)[U],
-                                           unsigned tag, X (&g)[U], int* err) {
+                                           unsigned tag, X (&g)[U], const LinkWait& wait) {
     LinkReg<X> r[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) r[u].set(v[u] == V(0) ? tag : ~tag);
@@ -175,10 +184,10 @@ __device__ __forceinline__ bool linkGather(const LinkCell<X>* __restrict__ x, co
         for (int u = 0; u < U; ++u) ready = ready && r[u].ready(tag);
         if (__all_sync(0xffffffffu, ready)) break;
         if constexpr (NAP > 0) __nanosleep(NAP);
-        if ((++polls & 1023) == 0) {
-            const bool out = polls >= kLinkPolls || *reinterpret_cast<volatile int*>(err) != 0;
+        if ((++polls & 1023) == 0 || polls >= wait.polls) {
+            const bool out = polls >= wait.polls || linkFailed(wait);
             if (__any_sync(0xffffffffu, out)) {
-                atomicExch(err, 1);
+                atomicExch(wait.err, 1);
                 return false;
             }
         }
@@ -193,7 +202,7 @@ __device__ __forceinline__ bool linkGather(const LinkCell<X>* __restrict__ x, co
 // one in sellDot's order, handed round by shuffles.
 template <int L, int NAP = 0, class V, class X>
 __device__ __forceinline__ double linkSellDot(const int* __restrict__ idx, const V* __restrict__ val, int2 h, int r,
-                                              int lane, const LinkCell<X>* x, unsigned tag, int* err, bool& ok) {
+                                              int lane, const LinkCell<X>* x, unsigned tag, const LinkWait& wait, bool& ok) {
     const int q = lane % L;
     const int* ip = idx + h.x + r;
     const V* vp = val + h.x + r;
@@ -209,7 +218,7 @@ __device__ __forceinline__ double linkSellDot(const int* __restrict__ idx, const
             c[u] = in ? __ldg(ip + k * kSlice) : 0;
             v[u] = in ? __ldg(vp + k * kSlice) : V(0);
         }
-        ok = linkGather<kLinkU, NAP>(x, c, v, tag, g, err) && ok;
+        ok = linkGather<kLinkU, NAP>(x, c, v, tag, g, wait) && ok;
 #pragma unroll
         for (int u = 0; u < kLinkU; ++u) {
             if (k0 + u * L >= h.y) break;  // the same in every lane
@@ -231,7 +240,7 @@ __device__ __forceinline__ double linkSellDot(const int* __restrict__ idx, const
 // added in warp order).  Every lane of a row's group returns its sum.
 template <int U, class V, class X>
 __device__ __forceinline__ double linkLaneSum(int b, int e, int first, int G, const int* __restrict__ idx,
-                                              const V* __restrict__ val, const LinkCell<X>* x, unsigned tag, int* err,
+                                              const V* __restrict__ val, const LinkCell<X>* x, unsigned tag, const LinkWait& wait,
                                               bool& ok) {
     double s[U];
 #pragma unroll
@@ -250,7 +259,7 @@ __device__ __forceinline__ double linkLaneSum(int b, int e, int first, int G, co
             c[u] = in ? __ldg(idx + k) : 0;
             v[u] = in ? __ldg(val + k) : V(0);
         }
-        ok = linkGather<W, kLinkNap>(x, c, v, tag, g, err) && ok;
+        ok = linkGather<W, kLinkNap>(x, c, v, tag, g, wait) && ok;
 #pragma unroll
         for (int u = 0; u < W; ++u) s[u % U] += static_cast<double>(v[u]) * static_cast<double>(g[u]);
     }
@@ -261,14 +270,14 @@ __device__ __forceinline__ double linkLaneSum(int b, int e, int first, int G, co
 }
 template <class V, class X>
 __device__ __forceinline__ double linkRowDot(int b, int e, int lane, int G, int U, const int* __restrict__ idx,
-                                             const V* __restrict__ val, const LinkCell<X>* x, unsigned tag, int* err,
+                                             const V* __restrict__ val, const LinkCell<X>* x, unsigned tag, const LinkWait& wait,
                                              bool& ok) {
     double t = 0.0;
     const int vw = G <= 32 ? 1 : G / 32;
     for (int w = 0; w < vw; ++w) {
         const int first = G <= 32 ? lane % G : w * 32 + lane;
-        double s = U == 8 ? linkLaneSum<8>(b, e, first, G, idx, val, x, tag, err, ok)
-                          : linkLaneSum<4>(b, e, first, G, idx, val, x, tag, err, ok);
+        double s = U == 8 ? linkLaneSum<8>(b, e, first, G, idx, val, x, tag, wait, ok)
+                          : linkLaneSum<4>(b, e, first, G, idx, val, x, tag, wait, ok);
         for (int off = min(G, 32) / 2; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
         t = w == 0 ? s : t + s;
     }
@@ -301,17 +310,17 @@ struct LinkArgs {
     IterArgs<T> it;
     LinkSide<T> P, D;  // columns (A^T), rows (A)
     LinkCell<T>*x, *y;
-    int* err;
+    LinkWait wait;
     LinkTime* time;
 };
 
 // Sum of this lane's row of unit u (L lanes per sliced-ELL row).
 template <int L, bool CSR, class T, class X>
 __device__ __forceinline__ double linkUnitDot(const LinkSide<T>& a, int u, int lane, const LinkCell<X>* x, unsigned tag,
-                                              int* err, bool& ok) {
+                                              const LinkWait& wait, bool& ok) {
     if (!CSR || (u >= a.nl && a.lanes == 0)) {
         const int v = u - a.nl;
-        return linkSellDot<L, CSR ? kLinkNap : 0>(a.idx, a.val, __ldg(a.hdr + v / L), v % L * (32 / L) + lane / L, lane, x, tag, err, ok);
+        return linkSellDot<L, CSR ? kLinkNap : 0>(a.idx, a.val, __ldg(a.hdr + v / L), v % L * (32 / L) + lane / L, lane, x, tag, wait, ok);
     }
     const bool lng = u < a.nl;
     const int G = lng ? a.llanes : a.lanes, W = lng ? a.lunroll : a.unroll;
@@ -319,7 +328,7 @@ __device__ __forceinline__ double linkUnitDot(const LinkSide<T>& a, int u, int l
     const int r = lng ? u : a.nl + (u - a.nl) * per + (per > 1 ? lane / G : 0);
     const bool in = r < a.rows;
     const int b = in ? __ldg(a.ptr + r) : 0, e = in ? __ldg(a.ptr + r + 1) : 0;
-    return linkRowDot(b, e, lane, G, W, a.cidx, a.cval, x, tag, err, ok);
+    return linkRowDot(b, e, lane, G, W, a.cidx, a.cval, x, tag, wait, ok);
 }
 // The row this lane updates of unit u (-1: none).
 template <int L, bool CSR, class T>
@@ -336,7 +345,8 @@ template <int LP, int LD, bool CSR, class T>
 __device__ __forceinline__ void linkedCycle(const LinkArgs<T>& a) {
     const IterArgs<T>& p = a.it;
     const DevState* st = p.st;
-    if (st->done || st->prec != precTag<T>()) return;
+    const bool failed = linkFailed(a.wait);
+    if (st->done || st->prec != precTag<T>() || failed) return;
     const int cur = st->phase == 0 ? st->total : st->polish_count;
     const int lim = st->phase == 0 ? p.max_iter : p.polish_max_iter;
     const int iters = min(p.N, lim - cur);
@@ -385,7 +395,7 @@ __device__ __forceinline__ void linkedCycle(const LinkArgs<T>& a) {
                 xi = static_cast<double>(p.xi[j]);
                 tau = step * static_cast<double>(q.tau) / pw;
             }
-            const double s = linkUnitDot<LP, CSR>(a.P, u, lane, a.y, tag - 1u, a.err, ok);
+            const double s = linkUnitDot<LP, CSR>(a.P, u, lane, a.y, tag - 1u, a.wait, ok);
             if (dclock && u == 0) dclk += clock64() - clk;
             if (j < 0) continue;
             double xh, xr;
@@ -405,7 +415,7 @@ __device__ __forceinline__ void linkedCycle(const LinkArgs<T>& a) {
                 ycd = p.yc[i];
                 yi = static_cast<double>(p.yi[i]);
             }
-            const double s = linkUnitDot<LD, CSR>(a.D, u, lane, a.x, tag, a.err, ok);
+            const double s = linkUnitDot<LD, CSR>(a.D, u, lane, a.x, tag, a.wait, ok);
             if (pclock && u == 0) pclk += clock64() - clk;
             if (i < 0) continue;
             double py;
