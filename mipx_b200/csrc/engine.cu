@@ -2461,9 +2461,15 @@ int32_t Engine::solveDevice(pdlpx_result* out) {
         step_ms_[p][0] = step_ms_[p][1] = 0.0;
         step_samples_[p] = 0;
     }
-    // A linked cycle is short beside the way to the host and back (25 us of 400-600),
-    // so the next one is queued before the state of the one at hand is read; once
-    // the solve has ended, what is queued returns at once.
+    // The way to the host and back takes 25 us beside a linked cycle's 400-600 at the
+    // default check frequency, so the next one is queued before the state of the one
+    // at hand is read; once the solve has ended, what is queued returns at once.  A
+    // stop request or a time limit then comes up to a cycle late, so this is done
+    // only while a cycle takes kAheadMs or less: where it takes longer the way to
+    // the host is below 0.5 % of it.  The first cycle is guessed at 16 us per
+    // iteration, the slowest measured.
+    constexpr double kAheadMs = 5.0;
+    double cycle_ms = 0.016 * N;
     struct Queued {
         int prec, link;
     } queue[2] = {};
@@ -2506,7 +2512,7 @@ int32_t Engine::solveDevice(pdlpx_result* out) {
             const int32_t rc = enqueue(want);
             if (rc != PDLPX_OK) return rc;
         }
-        if (want && queued == 1 && queue[head].link) {
+        if (want && queued == 1 && queue[head].link && cycle_ms <= kAheadMs) {
             const int32_t rc = enqueue(1);
             if (rc != PDLPX_OK) return rc;
         }
@@ -2525,6 +2531,7 @@ int32_t Engine::solveDevice(pdlpx_result* out) {
             const double clk = static_cast<double>(q.primal_clk + q.dual_clk);
             if (h.total > prev_total && q.iters > 0 && clk > 0.0) {
                 const double ms = 1e-6 * static_cast<double>(q.ns) / q.iters;
+                cycle_ms = ms * N;
                 step_ms_[ran][0] += ms * static_cast<double>(q.primal_clk) / clk;
                 step_ms_[ran][1] += ms * static_cast<double>(q.dual_clk) / clk;
                 ++step_samples_[ran];
