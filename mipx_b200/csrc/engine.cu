@@ -26,6 +26,7 @@
 #include "kernels.cuh"
 #include "anderson.cuh"
 #include "control.cuh"
+#include "link_plan.hpp"
 #include "linked.cuh"
 #include "shapes.cuh"
 #include "tiny.cuh"
@@ -615,7 +616,15 @@ struct DeviceLp {
     int link_warps = 0;  // of its grid per SM
     bool link_refused = false;  // its launch failed on this image: the step launches run
     int tiny = 0;        // one block runs it (tiny.cuh): 1 short columns, 2 short rows
-    int sell_max[2] = {0, 0};  // most entries of a sliced-ELL column / row
+    int longestRow[2] = {0, 0};  // entries of the longest column / row that is not one of the long ones
+    // Both forms tried (link_plan.hpp): whether to, and their time and iterations so
+    // far, [FP32 / FP64][step launches / linked]
+    bool link_try = false;
+    struct Tried {
+        double ms = 0.0;
+        int iters = 0;
+    } tried[2][2];
+    cudaEvent_t try_ev[2] = {nullptr, nullptr};
     void *link_x = nullptr, *link_y = nullptr;  // cells (null: the launches run)
 
     // [FP32 / FP64][step launches / linked]
@@ -633,13 +642,15 @@ struct DeviceLp {
     } key;
     void keepGraphsOf(const pdlpx_options& o) {
         if (key.N != o.termination_eval_frequency || key.max_iter != o.max_iter ||
-            key.polish_max_iter != o.polish_max_iter || key.link_polls != o.link_polls || key.aa_reg != o.anderson_regularization) {
-            for (auto& row : cycle)
-                for (auto& g : row) drop(g);
-        }
+            key.polish_max_iter != o.polish_max_iter || key.link_polls != o.link_polls || key.aa_reg != o.anderson_regularization)
+            dropCycles();
         if (key.sv_max_iter != o.sv_max_iter || key.sv_tol != o.sv_tol) drop(power);
         key = GraphKey{o.termination_eval_frequency, o.max_iter, o.polish_max_iter, o.link_polls, o.sv_max_iter,
                        o.anderson_regularization, o.sv_tol};
+    }
+    void dropCycles() {
+        for (auto& row : cycle)
+            for (auto& g : row) drop(g);
     }
     static void drop(cudaGraphExec_t& g) {
         if (g) cudaGraphExecDestroy(g);
@@ -647,8 +658,7 @@ struct DeviceLp {
     }
 
     ~DeviceLp() {
-        for (auto& row : cycle)
-            for (auto& g : row) drop(g);
+        dropCycles();
         for (auto& row : kev)
             for (auto& e : row)
                 if (e) cudaEventDestroy(e);
@@ -656,6 +666,8 @@ struct DeviceLp {
         if (arena) cudaFree(arena);
         if (h_sb) cudaFreeHost(h_sb);
         for (auto& e : copied)
+            if (e) cudaEventDestroy(e);
+        for (auto& e : try_ev)
             if (e) cudaEventDestroy(e);
         if (h_ps) cudaFreeHost(h_ps);
         if (stream) cudaStreamDestroy(stream);
@@ -1003,35 +1015,13 @@ LinkSide<T> linkSide(const DeviceLp& d, const IterArgs<T>& ia, bool primal) {
     return a;
 }
 
-// Whether the linked cycle runs the steps of an LP, and with how many lanes per
-// sliced-ELL column (link_lanes).  Measured on B200 (us per iteration with check,
-// restart and power iteration, launches -> linked; random LPs have 8 entries per
-// column and 20 per row):
-//  * sliced ELL on both sides: 400 x 1,000 7.9 -> 3.3, 2,000 x 5,000 9.0 -> 4.3,
-//    20,000 x 50,000 14.2 -> 12.3, 30,000 x 75,000 (600k entries) 17.5 -> 15.5,
-//    40,000 x 100,000 23.0 -> 22.5: up to 600k entries.  4 lanes per column (8 per
-//    row) to 240k entries (12,000 x 30,000 9.6 against 10.0 with 2 and 4), above
-//    that 2 (20,000 x 50,000 12.3 against 14.1: more warps than an SM holds).
-//    Columns of up to 3 entries take one lane (transportation 30 x 40: 2.6
-//    against 2.8), long ones 8.
-//  * long rows beside sliced ELL (power law, launches with long and short columns
-//    in one): columns of up to 500 entries at 1,000 x 4,000 14.9 -> 6.9, 4,000 x
-//    16,000 16.0 -> 13.4, 8,000 x 32,000 (317k entries) 17.7 -> 15.8, up to 1,000
-//    at 2,000 x 8,000 16.0 -> 9.5, but up to 2,000 at 4,000 x 16,000 16.4 -> 19.1
-//    (one warp sums a long row): to 350k entries and rows of 1,000.
-//  * a CSR side: transportation 97 x 131 (25k entries) 5.7 -> 3.3, 150 x 150 5.7 ->
-//    4.7, 200 x 200 (80k) 5.5 -> 5.4, 250 x 250 5.8 -> 6.4: to 90k.
-//  * one block takes an LP whose slices are its warps and whose entries fit their
-//    registers (tiny.cuh): 90 x 250 linked 2.3 -> 1.2.  No block waits on another,
-//    so it needs no share of the SMs (link_warps 0).
-// Options that pin a launch shape keep the launches.
+// Whether the linked cycle may run the steps of an LP (link_plan.hpp has the rest of
+// the rule): its image then holds the cells.  Options that pin a launch shape keep
+// the launches.
 bool linkCsr(const DeviceLp& d) { return !isSell(d.shapeP) || !isSell(d.shapeD) || d.nlP > 0 || d.nlD > 0; }
 bool linkable(const DeviceLp& d, const pdlpx_options& o) {
-    if (d.lt_C > 0 || o.hot_cache > 0) return false;
-    if (o.shape_primal > 0 || o.shape_dual > 0 || o.spmv_group_a > 0 || o.spmv_group_at > 0) return false;
-    const bool csr = !isSell(d.shapeP) || !isSell(d.shapeD);
-    if (d.longest > 1000) return false;
-    return d.nnz <= (csr ? 90000 : (d.nlP > 0 || d.nlD > 0) ? 350000 : 600000);
+    return d.lt_C == 0 && o.hot_cache <= 0 && o.shape_primal <= 0 && o.shape_dual <= 0 && o.spmv_group_a <= 0 &&
+           o.spmv_group_at <= 0 && d.nnz <= kLinkEntries;
 }
 // f(kernel, lanes per sliced-ELL column, lanes per sliced-ELL row) of the planned grid.
 template <class T, class F>
@@ -1050,30 +1040,52 @@ int linkedUnits(const DeviceLp& d, bool primal, int sub) {
 }
 int linkedGrid(const DeviceLp& d, int units) { return std::min(d.sms, (units + d.link_warps - 1) / d.link_warps); }
 
+// Whether and how the linked cycle runs the steps.  Lanes per sliced-ELL column: 4 (8
+// per row) to 240k entries (12,000 x 30,000 9.6 us per iteration against 10.0 with 2
+// and 4), above that 2 (20,000 x 50,000 12.3 against 14.1: more warps than an SM
+// holds); columns of up to 3 entries take one lane (transportation 30 x 40: 2.6
+// against 2.8), long ones 8.  One block takes an LP whose slices are its warps and
+// whose entries fit their registers (tiny.cuh): 90 x 250 linked 2.3 -> 1.2.  No block
+// waits on another there, so it needs no share of the SMs (link_warps 0).
 void planLinked(DeviceLp& d) {
     // rowDotU with two sums per lane (the autotuner may pick it) has no linked form
     auto supported = [](int shape) { return isSell(shape) || kShapes[shape].U >= kLinkU; };
     d.linked = d.link_x != nullptr && !d.link_refused && supported(d.shapeP) && supported(d.shapeD);
     d.tiny = d.link_warps = 0;
+    d.link_try = false;
     if (!d.linked) return;
     if (!linkCsr(d) && (d.n + kSlice - 1) / kSlice + (d.m + kSlice - 1) / kSlice <= kTinyWarps) {
-        if (d.sell_max[0] <= kTinyShort && d.sell_max[1] <= kTinyLong)
+        if (d.longestRow[0] <= kTinyShort && d.longestRow[1] <= kTinyLong)
             d.tiny = 1;
-        else if (d.sell_max[0] <= kTinyLong && d.sell_max[1] <= kTinyShort)
+        else if (d.longestRow[0] <= kTinyLong && d.longestRow[1] <= kTinyShort)
             d.tiny = 2;
     }
     if (d.tiny != 0) return;
     const double mean = static_cast<double>(d.nnz - d.zlP) / std::max(1, d.n - d.nlP);
     d.link_lanes = mean <= 3.0 ? 1 : mean > 14.0 ? 8 : d.nnz <= 240000 ? 4 : 2;
+    LinkShape shape;
+    shape.nnz = d.nnz;
+    shape.longest = d.longest;
+    auto side = [&](bool primal, int sub) {
+        const int sh = primal ? d.shapeP : d.shapeD;
+        return LinkSideShape{primal ? d.n : d.m, primal ? d.nlP : d.nlD, isSell(sh) ? 0 : kShapes[sh].G,
+                             d.longestRow[primal ? 0 : 1], linkedUnits(d, primal, sub)};
+    };
     // one warp per unit over all SMs first (a unit's gathers queue in its SM's
     // L1), and no wider blocks than that takes: small LPs leave room for the
     // grids of other solvers
     auto plan = [&](auto kernel, int lp, int ld) {
-        const int units = linkedUnits(d, true, lp) + linkedUnits(d, false, ld);
+        shape.P = side(true, lp);
+        shape.D = side(false, ld);
+        const int units = shape.P.units + shape.D.units;
         d.link_warps = std::min(linkThreads(linkCsr(d)) / 32, (units + d.sms - 1) / d.sms);
+        shape.warps = d.sms * d.link_warps;
         return cooperativeFits(kernel, d.device, d.sms, linkedGrid(d, units), 32 * d.link_warps);
     };
     d.linked = withLinked<double>(d, plan) && (!d.mixed || withLinked<float>(d, plan));
+    const LinkRule rule = linkRule(shape);
+    if (rule == LinkRule::kNever) d.linked = false;
+    d.link_try = rule == LinkRule::kTry;
     if (!d.linked) d.link_warps = 0;
 }
 
@@ -1591,8 +1603,6 @@ static int32_t buildDevice(std::unique_ptr<DeviceLp>& dp, const ScaledLp& sc_in,
     SellHost hsP, hsD;
     if (sellP && !buildSell(sc.at, d.nlP, hsP)) sellP = false;
     if (sellD && !buildSell(sc.a, d.nlD, hsD)) sellD = false;
-    for (const int2& h : hsP.hdr) d.sell_max[0] = std::max(d.sell_max[0], h.y);
-    for (const int2& h : hsD.hdr) d.sell_max[1] = std::max(d.sell_max[1], h.y);
     const auto tbs = std::chrono::steady_clock::now();
     d.m = sc.a.rows;
     d.n = sc.a.cols;
@@ -1603,6 +1613,10 @@ static int32_t buildDevice(std::unique_ptr<DeviceLp>& dp, const ScaledLp& sc_in,
     d.zlD = zlD;
     d.zlP = zlP;
     d.longest = std::max(d.nlD > 0 ? sc.a.ptr[1] : 0, d.nlP > 0 ? sc.at.ptr[1] : 0);  // the longest come first
+    if (nnz <= kLinkEntries) {
+        for (int32_t j = d.nlP; j < d.n; ++j) d.longestRow[0] = std::max(d.longestRow[0], sc.at.ptr[j + 1] - sc.at.ptr[j]);
+        for (int32_t i = d.nlD; i < d.m; ++i) d.longestRow[1] = std::max(d.longestRow[1], sc.a.ptr[i + 1] - sc.a.ptr[i]);
+    }
     LongTilesHost ltH;
     // automatic: when the long columns hold at least 1.5 times as many entries
     // per SM as a chunk has rows (each tile's copy of y then serves >= 1.5
@@ -1720,6 +1734,7 @@ static int32_t buildDevice(std::unique_ptr<DeviceLp>& dp, const ScaledLp& sc_in,
     PDLPX_CK(cudaMallocHost(reinterpret_cast<void**>(&d.h_sb), 2 * sizeof(StateBlock)));
     d.h_st = &d.h_sb[0].st;
     for (auto& e : d.copied) PDLPX_CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    for (auto& e : d.try_ev) PDLPX_CK(cudaEventCreate(&e));
     PDLPX_CK(cudaMallocHost(reinterpret_cast<void**>(&d.h_ps), sizeof(PowerState)));
     char* b = d.arena;
     d.a_ptr = reinterpret_cast<int*>(b + o_a_ptr);
@@ -2266,6 +2281,9 @@ int32_t Engine::solveDevice(pdlpx_result* out) {
         const int32_t rc = d.mixed ? autotuneShapes<float>(d, opt_, tp, td, err)
                                    : autotuneShapes<double>(d, opt_, tp, td, err);
         if (rc != PDLPX_OK) return rc;
+        d.dropCycles();  // of the shapes before
+        for (auto& row : d.tried)
+            for (auto& t : row) t = DeviceLp::Tried{};
     }
     const int32_t m = lp_.m, n = lp_.n;
     const int N = opt_.termination_eval_frequency;
@@ -2470,6 +2488,24 @@ int32_t Engine::solveDevice(pdlpx_result* out) {
     // iteration, the slowest measured.
     constexpr double kAheadMs = 5.0;
     double cycle_ms = 0.016 * N;
+    // Where it is not known whether the linked cycle pays: one cycle of each form (or
+    // as many as make kTryIters iterations), then the faster one, kept with the image.
+    // Not while a cycle is long (the wrong one would cost as much) -- the launches run.
+    constexpr int kTryIters = 100;
+    auto undecided = [&] {
+        return d.linked && d.link_try &&
+               (d.tried[prec][0].iters < kTryIters || d.tried[prec][1].iters < kTryIters);
+    };
+    auto pickLinked = [&]() -> int {
+        if (!d.linked) return 0;
+        if (d.tiny != 0) return 1;
+        if (!link_share.fits()) return 0;
+        if (!d.link_try) return 1;
+        const DeviceLp::Tried &a = d.tried[prec][0], &b = d.tried[prec][1];
+        if (!undecided()) return b.ms / b.iters < a.ms / a.iters ? 1 : 0;
+        if (cycle_ms > kAheadMs) return 0;
+        return b.iters < kTryIters ? 1 : 0;
+    };
     struct Queued {
         int prec, link;
     } queue[2] = {};
@@ -2482,7 +2518,7 @@ int32_t Engine::solveDevice(pdlpx_result* out) {
         cudaStream_t s;
         ~Drain() { cudaStreamSynchronize(s); }
     } drain{s};
-    auto enqueue = [&](int link) -> int32_t {
+    auto enqueue = [&](int link, bool timed) -> int32_t {
         cudaError_t e = ensureCycle(prec, link);
         if (e != cudaSuccess && link) {  // the same bits by launches
             d.link_refused = true;
@@ -2493,7 +2529,12 @@ int32_t Engine::solveDevice(pdlpx_result* out) {
         }
         PDLPX_CK(e);
         const int slot = (head + queued) & 1;
+        if (timed) {
+            PDLPX_CK(cudaGraphUpload(d.cycle[prec][link], s));
+            PDLPX_CK(cudaEventRecord(d.try_ev[0], s));
+        }
         PDLPX_CK(cudaGraphLaunch(d.cycle[prec][link], s));
+        if (timed) PDLPX_CK(cudaEventRecord(d.try_ev[1], s));
         launches += d.launches_cycle[prec][link];
         PDLPX_CK(cudaMemcpyAsync(&d.h_sb[slot], d.st, sizeof(StateBlock), cudaMemcpyDeviceToHost, s));
         PDLPX_CK(cudaEventRecord(d.copied[slot], s));
@@ -2507,13 +2548,14 @@ int32_t Engine::solveDevice(pdlpx_result* out) {
             stopped = true;
             break;
         }
-        const int want = d.linked && (d.tiny != 0 || link_share.fits()) ? 1 : 0;
+        const int want = pickLinked();
+        const bool timed = queued == 0 && undecided();
         if (queued == 0) {
-            const int32_t rc = enqueue(want);
+            const int32_t rc = enqueue(want, timed);
             if (rc != PDLPX_OK) return rc;
         }
-        if (want && queued == 1 && queue[head].link && cycle_ms <= kAheadMs) {
-            const int32_t rc = enqueue(1);
+        if (want && !timed && queued == 1 && queue[head].link && cycle_ms <= kAheadMs) {
+            const int32_t rc = enqueue(1, false);
             if (rc != PDLPX_OK) return rc;
         }
         PDLPX_CK(cudaEventSynchronize(d.copied[head]));
@@ -2525,6 +2567,12 @@ int32_t Engine::solveDevice(pdlpx_result* out) {
         if (block.link_err != 0) {
             err = "linked cycle: a wait ran out of polls";
             return PDLPX_E_TIMEOUT;
+        }
+        if (timed && h.total > prev_total) {
+            float ms = 0.0f;
+            PDLPX_CK(cudaEventElapsedTime(&ms, d.try_ev[0], d.try_ev[1]));
+            d.tried[ran][link].ms += ms;
+            d.tried[ran][link].iters += h.total - prev_total;
         }
         if (link) {
             const LinkTime& q = block.lt;

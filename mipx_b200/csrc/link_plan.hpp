@@ -1,0 +1,82 @@
+// Which LPs' steps the linked restart cycle (linked.cuh) runs.  Host only.
+//
+// The linked cycle and the step launches give the same bits, so the choice is one
+// of speed alone.  Measured on B200 (us per iteration with the check, launches ->
+// linked, 190 random, transportation and power-law LPs):
+//  * Sliced ELL on both sides: 1.2-3.4 times as fast up to 150k entries (400 x
+//    1,000 7.9 -> 3.3, 2,000 x 5,000 9.0 -> 4.3, 42k x 40k of 120k 7.3 -> 6.2), but
+//    57k x 32k rows 6.8 -> 6.9.  Up to 600k it depends on the LP: 30k x 51k of 308k
+//    10.3 -> 6.4, 6k x 29k of 322k 13.9 -> 20.1, 25k x 29k of 630k 14.7 -> 14.1.
+//  * Long rows beside sliced ELL (power law), a warp each: up to 50k entries and
+//    rows of 512 14.4 -> 9.4 and better; beyond 1,756 x 8,375 of 83k 18.0 -> 11.9,
+//    but 4,203 x 6,843 of 65k 13.6 -> 14.2 and every LP of 420k or more slower.
+//  * A CSR side.  Every row of it gathers the same few values, and the warps polling
+//    their lines of L2 hold up the stores to them: what decides is the loads per
+//    line (crowd).  Up to 1,000, with one round of loads per row and one unit per
+//    warp, transportation 70 x 70 5.2 -> 3.0, 97 x 131 4.4 -> 3.4, 70 x 300 6.4 ->
+//    4.0; 150 x 150 (1,200) 5.5 -> 5.1, 200 x 200 (1,600) 5.5 -> 6.8, 300 x 100
+//    between 0.9 and 1.1 times as fast from run to run.  Both sides crowded, 398 x
+//    318 dense 5.8 -> 10.7; 143 x 7,113 (4,400) 7.3 -> 15.0; more than two units per
+//    warp, 35,834 x 488 6.6 -> 16.9; long rows besides, power law 12-15 -> 16-28.
+//    Above that crowd it pays only where the launches walk long sliced-ELL columns,
+//    97 x 1,752 dense 12.6 -> 7.9.
+// Between the sure cases and the hopeless ones the engine tries both (kTry): a cycle
+// of each, then the faster one.
+#pragma once
+
+#include <algorithm>
+#include <cstdint>
+
+namespace pdlpx {
+
+struct LinkSideShape {
+    int rows = 0;
+    int nl = 0;        // long rows among them, in CSR
+    int lanes = 0;     // of the others: 0 sliced ELL, else CSR lanes per row
+    int longest = 0;   // entries of the longest of the others
+    int units = 0;     // linkUnits
+};
+struct LinkShape {
+    std::int64_t nnz = 0;
+    int longest = 0;   // entries of the longest of the long rows
+    int warps = 0;     // of the grid
+    LinkSideShape P, D;  // columns, rows
+};
+
+constexpr std::int64_t kLinkEntries = 600000;  // no LP beyond
+
+enum class LinkRule { kNever, kTry, kAlways };
+
+// Rounds of eight loads per lane that a warp takes for a CSR row (linkRowDot).
+inline int linkRounds(int longest, int lanes) {
+    return std::max(1, lanes / 32) * ((longest + 8 * lanes - 1) / (8 * lanes));
+}
+
+inline LinkRule linkRule(const LinkShape& s) {
+    const bool csr = s.P.lanes > 0 || s.D.lanes > 0, longs = s.P.nl > 0 || s.D.nl > 0;
+    if (s.longest > 1000) return LinkRule::kNever;
+    if (!csr && !longs) {
+        if (s.nnz <= 150000 && s.P.rows + s.D.rows <= 60000) return LinkRule::kAlways;
+        return s.nnz <= kLinkEntries ? LinkRule::kTry : LinkRule::kNever;
+    }
+    if (!csr) {
+        if (s.nnz <= 50000 && s.longest <= 512) return LinkRule::kAlways;
+        return s.nnz <= 350000 ? LinkRule::kTry : LinkRule::kNever;
+    }
+    if (longs || s.nnz > 90000) return LinkRule::kNever;
+    int rounds = 1, serial = 0, per_warp = 1;
+    for (const LinkSideShape* a : {&s.P, &s.D}) {
+        if (a->lanes > 0)
+            rounds = std::max(rounds, linkRounds(a->longest, a->lanes));
+        else
+            serial = std::max(serial, a->longest);
+        per_warp = std::max(per_warp, (a->units + s.warps - 1) / std::max(1, s.warps));
+    }
+    // loads of x (by the rows) and of y (by the columns) per line of eight cells
+    const std::int64_t x = 8 * s.nnz / std::max(1, s.P.rows), y = 8 * s.nnz / std::max(1, s.D.rows);
+    if (x + y <= 1000 && rounds == 1 && per_warp == 1 && s.nnz <= 50000) return LinkRule::kAlways;
+    if (per_warp > 2 || rounds > 8 || std::min(x, y) > 500) return LinkRule::kNever;
+    return x + y <= 2500 || serial >= 32 ? LinkRule::kTry : LinkRule::kNever;
+}
+
+}  // namespace pdlpx
