@@ -28,7 +28,7 @@
 // -> FP64 hand-overs and the tile modes -- is one CUDA graph launch.  When
 // finished LPs leave enough tiles idle, the host switches the launches to a
 // list of the live tiles and captures a smaller graph.  While the live LPs of a
-// sliced-ELL pack are few (kLinkPackEntries) their steps run as one linked cycle
+// sliced-ELL pack are few (linkPackLanes) their steps run as one linked cycle
 // instead (linked.cuh), with the same bits.
 //
 // An LP's tiles, launch shape, storage and reduction order depend on that LP
@@ -52,6 +52,7 @@
 #include "control.cuh"
 #include "engine.hpp"
 #include "kernels.cuh"
+#include "link_plan.hpp"
 #include "linked.cuh"
 #include "pack.hpp"
 #include "shapes.cuh"
@@ -329,13 +330,6 @@ struct LinkPackArgs {
     int np, nd, N;
 };
 constexpr int kLinkPackThreads = 512;
-// Live entries up to which the linked cycle runs a pack's steps.  Measured on
-// B200 (ms per batch_solve, launches -> linked): 12 LPs of 118k entries in FP64
-// 187 -> 88, 6 of 454k 69 -> 56; 64 LPs of 2.1M entries 280 with launches, 362
-// linked throughout, and 254 linked once the live LPs are down to 1M (266 from
-// 400k on).
-constexpr int64_t kLinkPackEntries = 1000000;
-
 __global__ void packLinkBegin(PackArgs a, LinkPackArgs q) {
     const int l = blockIdx.x * blockDim.x + threadIdx.x;
     if (l >= a.L) return;
@@ -1221,15 +1215,16 @@ struct Pack {
         linked = false;
         link_warps = 0;
         if (!linkable) return cudaSuccess;
-        int64_t z = 0, units = 0;
+        int64_t z = 0, units4 = 0, units2 = 0;  // with 4 lanes per column and 8 per row; 2 and 4
         for (const Item* it : items)
             if (keep[it->l]) {
                 z += it->sc.a.nnz();
-                units += (it->lp.n + 7) / 8 + (it->lp.m + 3) / 4;
+                units4 += (it->lp.n + 7) / 8 + (it->lp.m + 3) / 4;
+                units2 += (it->lp.n + 15) / 16 + (it->lp.m + 7) / 8;
             }
-        if (z > kLinkPackEntries || units == 0) return cudaSuccess;
         const int warps_max = kLinkPackThreads / 32;
-        link_lanes = units <= 3 * static_cast<int64_t>(sms) * warps_max ? 4 : 2;
+        link_lanes = linkPackLanes(z, units4, units2, static_cast<int64_t>(sms) * warps_max);
+        if (link_lanes == 0) return cudaSuccess;
         const int rc = kSlice / link_lanes, rr = kSlice / (2 * link_lanes);
         h_pu.clear();
         h_du.clear();

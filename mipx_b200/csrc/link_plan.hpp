@@ -79,4 +79,21 @@ inline LinkRule linkRule(const LinkShape& s) {
     return x + y <= 2500 || serial >= 32 ? LinkRule::kTry : LinkRule::kNever;
 }
 
+// A pack of sliced-ELL LPs: lanes per column (twice as many per row) of its linked
+// cycle, 0 where the step launches run.  units4, units2: units of the live LPs with 4
+// lanes per column (8 per row), with 2; warps: the most the grid has.  What decides is
+// the units a warp walks one after another.  Measured on B200 (us per iteration in
+// FP64, launches -> linked): 300 LPs of 50 x 125 (278k entries, 1.8 units per warp)
+// 13.7 -> 7.9, 2 of 15,000 x 40,000 (640k, 3.7) 17.9 -> 15.1, but 3 (960k, 5.5) 19.4
+// -> 20.8, 100 of 1,000 x 300 (741k, 6.1) 14.6 -> 18.4, 20 of 5,000 x 20,000 with one
+// or two entries per column (600k, 15.8) 18.8 -> 30.4, 6 and 20 of 20,000 x 5,000
+// (120k, 7.1 and 400k, 23.8) 11.1 -> 12.3 and 14.7 -> 37.9.  Batches, whose live LPs
+// become fewer: 64 LPs (2.1M entries, ms per call) 274 by launches, 242-248 linked
+// from 4.5 or 5.5 units per warp on, 257 from 3.5 on; 24 LPs in FP64 181 -> 121.
+inline int linkPackLanes(std::int64_t nnz, std::int64_t units4, std::int64_t units2, std::int64_t warps) {
+    const int lanes = units4 <= 3 * warps ? 4 : 2;
+    const std::int64_t units = lanes == 4 ? units4 : units2;
+    return units > 0 && 2 * units <= 9 * warps && nnz <= 1000000 ? lanes : 0;
+}
+
 }  // namespace pdlpx

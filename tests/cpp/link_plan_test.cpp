@@ -29,7 +29,26 @@ static void expect(LinkRule want, const char* name, long long nnz, int m, int n,
     ++bad;
 }
 
+// `count` LPs of m x n with `nnz` entries each, all live
+static void pack(int want, const char* name, long long count, int m, int n, long long nnz) {
+    const long long u4 = count * ((n + 7) / 8 + (m + 3) / 4), u2 = count * ((n + 15) / 16 + (m + 7) / 8);
+    const int got = linkPackLanes(count * nnz, u4, u2, 148 * 16);
+    if (got == want) return;
+    std::printf("FAIL pack %s: %d instead of %d\n", name, got, want);
+    ++bad;
+}
+
 int main() {
+    pack(0, "no LP", 0, 50, 125, 930);
+    pack(4, "12 of 1,000 x 2,500", 12, 1000, 2500, 20000);
+    pack(2, "300 of 50 x 125", 300, 50, 125, 930);
+    pack(0, "800 of 50 x 125", 800, 50, 125, 930);
+    pack(2, "2 of 15,000 x 40,000", 2, 15000, 40000, 320000);
+    pack(0, "3 of 15,000 x 40,000", 3, 15000, 40000, 320000);
+    pack(0, "100 of 1,000 x 300", 100, 1000, 300, 7410);
+    pack(0, "20 of 5,000 x 20,000", 20, 5000, 20000, 30000);
+    pack(0, "6 of 20,000 x 5,000", 6, 20000, 5000, 19900);
+    pack(0, "entries", 1, 1000, 1000, 1000001);
     const auto never = LinkRule::kNever, maybe = LinkRule::kTry, always = LinkRule::kAlways;
     // sliced ELL on both sides
     expect(always, "400 x 1,000", 8000, 400, 1000, 0, 0, 12, 35, 4, 8);
