@@ -881,7 +881,7 @@ struct Pack {
     std::vector<int> h_cl, h_rl;       // host copies of the live-tile lists
     PackArgs args{};
     // linked cycle: cells and unit lists of the live LPs
-    bool linkable = false;       // every side is sliced ELL
+    bool linkable = false;       // every side is sliced ELL and no option pins its launch shape
     bool linked = false;         // the live LPs are few enough
     int link_lanes = 4, link_warps = 0;
     cudaGraphExec_t lcycle = nullptr;
@@ -911,7 +911,7 @@ struct Pack {
 
     // Positions: columns grouped by primal shape, rows by dual shape, LP order
     // within a shape; each LP padded to whole tiles.
-    void place() {
+    void place(const pdlpx_options& o) {
         for (int side = 0; side < 2; ++side) {
             int64_t pos = 0, z = 0, ent = 0, sell_rows = 0;
             int tiles = 0;
@@ -961,7 +961,7 @@ struct Pack {
         listed = false;
         live_ct = nct;
         live_rt = nrt;
-        linkable = true;
+        linkable = o.shape_primal <= 0 && o.shape_dual <= 0 && o.spmv_group_a <= 0 && o.spmv_group_at <= 0;
         for (const Item* it : items) linkable = linkable && isSell(it->shapeP) && isSell(it->shapeD);
     }
 
@@ -1704,7 +1704,7 @@ int32_t solvePack(Pack& pk, const pdlpx_options& o, std::chrono::steady_clock::t
                   const std::atomic<int>* stop, const LpDone& done, std::string& err) {
     const int L = pk.L;
     for (int l = 0; l < L; ++l) pk.items[l]->l = l;
-    pk.place();
+    pk.place(o);
     pk.layout();
     bool any_warm = false;
     for (const Item* it : pk.items) any_warm |= !it->warm_x.empty();
