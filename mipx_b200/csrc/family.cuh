@@ -282,33 +282,6 @@ __device__ __forceinline__ void cutColumn(const FamArgs& a, int j, int l, bool o
         famCutColumns<1, false>(a, j, 1, l, on, add);
 }
 
-// Dual proximal step of one row (pdlp_kernels.cu:94-157, as dualUpdate) given
-// s = (A_l x_refl)_i; returns the new current y, py the pdhg y.
-__device__ __forceinline__ double famDualStep(const RowPack<double>& q, double yc, double yi, double s, double step,
-                                              double pw, double lam, double& py) {
-    const double sig = step * q.sigma * pw;
-    const double v = yc + sig * s;
-    const int type = static_cast<int>(q.type);
-    if (type == 0) {
-        py = v - sig * q.rl;
-    } else if (type == 1) {
-        py = v - sig * q.ru;
-        if (py < 0.0) py = 0.0;
-    } else if (type == 2) {
-        py = v - sig * q.rl;
-        if (py > 0.0) py = 0.0;
-    } else {
-        if (v >= sig * q.ru)
-            py = v - sig * q.ru;
-        else if (v <= sig * q.rl)
-            py = v - sig * q.rl;
-        else
-            py = 0.0;
-    }
-    const double yr = 2.0 * py - yc;
-    return lam * yr + (1.0 - lam) * yi;
-}
-
 // ---- PDHG step -----------------------------------------------------------------
 // Primal: one warp per R consecutive columns;
 // (A_l^T y)_j = c_lj (sum_i a_ij ys_il + appended entries).  Lanes of LPs
@@ -349,11 +322,8 @@ __global__ void __launch_bounds__(kBlock, 4) famPrimal(FamArgs a, int koff) {
         const ColPack<double> c = a.cp[q];
         const double cs = a.cs[q], xc = a.xc[q], xi = a.xi[q];
         const double tau = step * c.tau / pw;
-        double xh = xc - tau * (c.c + cs * s[r]);
-        if (xh < c.lb) xh = c.lb;
-        if (xh > c.ub) xh = c.ub;
-        const double xr = 2.0 * xh - xc;
-        a.xc[q] = lam * xr + (1.0 - lam) * xi;
+        double xh, xr;
+        a.xc[q] = primalAlong<double>(c, xc, xi, __fma_rn(cs, s[r], c.c), tau, lam, xh, xr);
         a.xs[q] = cs * xr;
         if (last) a.xh[q] = xh;
     }
@@ -395,7 +365,7 @@ __global__ void __launch_bounds__(kBlock, 4) famDual(FamArgs a, int koff) {
             const size_t q = fIdx(i0 + r, l);
             const double rs = a.rs[q], yc = a.yc[q];
             double py;
-            const double yn = famDualStep(a.rp[q], yc, a.yi[q], rs * s[r], step, pw, lam, py);
+            const double yn = dualValues<double>(a.rp[q], yc, a.yi[q], rs * s[r], step, pw, lam, py);
             a.yc[q] = yn;
             a.ys[q] = rs * yn;
             if (last) a.yh[q] = py;
@@ -415,7 +385,7 @@ __global__ void __launch_bounds__(kBlock, 4) famDual(FamArgs a, int koff) {
     const double lam = static_cast<double>(kk) / static_cast<double>(kk + 1);
     const double rs = a.rs[q], yc = a.yc[q];
     double py;
-    const double yn = famDualStep(a.rp[q], yc, a.yi[q], rs * s, st->step, st->pw, lam, py);
+    const double yn = dualValues<double>(a.rp[q], yc, a.yi[q], rs * s, st->step, st->pw, lam, py);
     a.yc[q] = yn;
     a.ys[q] = rs * yn;
     if (last) a.yh[q] = py;

@@ -401,19 +401,25 @@ __device__ __forceinline__ double average(double lam, double r, double a) {
     return __fma_rn(1.0 - lam, a, __dmul_rn(lam, r));
 }
 
-// Values of the Halpern primal step of a column given s = (A^T y_cur)_j:
+// Values of the Halpern primal step of a column given g = (c + A^T y_cur)_j:
 // projected gradient step (xh), reflection (xr), averaging with the anchor
 // (returned: the new current x) (pdlp_kernels.cu:46-88).  FP64 arithmetic with
 // the reference's association (tau = step * tau_base / omega).
 template <class T>
-__device__ __forceinline__ double primalValues(const ColPack<T>& q, double xcd, double xid, double s, double tau,
-                                               double lam, double& xh, double& xr) {
-    xh = __fma_rn(-tau, static_cast<double>(q.c) + s, xcd);
+__device__ __forceinline__ double primalAlong(const ColPack<T>& q, double xcd, double xid, double g, double tau,
+                                              double lam, double& xh, double& xr) {
+    xh = __fma_rn(-tau, g, xcd);
     const double lb = q.lb, ub = q.ub;
     if (xh < lb) xh = lb;
     if (xh > ub) xh = ub;
     xr = 2.0 * xh - xcd;
     return average(lam, xr, xid);
+}
+// given s = (A^T y_cur)_j
+template <class T>
+__device__ __forceinline__ double primalValues(const ColPack<T>& q, double xcd, double xid, double s, double tau,
+                                               double lam, double& xh, double& xr) {
+    return primalAlong<T>(q, xcd, xid, __dadd_rn(static_cast<double>(q.c), s), tau, lam, xh, xr);
 }
 
 template <class T>
