@@ -62,7 +62,7 @@ struct FamArgs {
     const int* k_lane;    // LP of each appended row
     const int* k_first;   // [33] first appended row of each lane
     const int* kt_ptr;    // appended entries by column: row, LP, value
-    const int* kt_lptr;   // [n * 32 + 1] the same entries by column and lane
+    const int* kt_lptr;   // [n * 32 + 1] the same entries by column and lane (listed)
     const int* kt_row;
     const int* kt_lane;
     const double* kt_val;
@@ -862,13 +862,19 @@ void famLaneData(const Item& it, int n, FamLaneData& q) {
 
 // The appended rows of the lanes in use (lane order; a lane without a member
 // contributes none): row pointers, entries, lanes, per-lane first row, and the
-// same entries by column and lane (row order inside both).
+// same entries by column (lane order, row order inside), with the bounds of every
+// lane's where the kernels walk them so (famListed; 32 times the columns' bounds,
+// 6.4 MB at 50,000 columns, otherwise built and uploaded at every admission for
+// nothing).
 struct FamCuts {
     std::vector<int32_t> kp, ki, kl, kf, ktp, ktlp, ktr, ktl;
     std::vector<double> kv, ktv;
     int K = 0;
     int64_t Zk = 0;
 };
+
+// Whether the kernels walk the appended entries by lane (famCutColumns).
+bool famListed(int64_t zk, int n) { return zk >= static_cast<int64_t>(kFamListed) * n; }
 
 void famBuildCuts(const FamPack& fp, const std::vector<char>& in_use, FamCuts& c) {
     const int n = fp.n, mb = fp.mb;
@@ -877,7 +883,6 @@ void famBuildCuts(const FamPack& fp, const std::vector<char>& in_use, FamCuts& c
     c.kv.clear();
     c.kl.clear();
     c.kf.assign(kFam + 1, 0);
-    std::vector<int32_t> colcnt(static_cast<size_t>(n) * kFam + 1, 0);
     int q = 0;
     for (int l = 0; l < kFam; ++l) {
         c.kf[l] = q;
@@ -889,7 +894,6 @@ void famBuildCuts(const FamPack& fp, const std::vector<char>& in_use, FamCuts& c
             for (int32_t k = a.ptr[i]; k < a.ptr[i + 1]; ++k) {
                 c.ki.push_back(a.idx[k]);
                 c.kv.push_back(a.val[k]);
-                ++colcnt[static_cast<size_t>(a.idx[k]) * kFam + l + 1];
             }
         }
     }
@@ -897,16 +901,23 @@ void famBuildCuts(const FamPack& fp, const std::vector<char>& in_use, FamCuts& c
     c.K = q;
     c.Zk = static_cast<int64_t>(c.ki.size());
     c.kp.push_back(static_cast<int32_t>(c.Zk));
-    for (size_t j = 1; j < colcnt.size(); ++j) colcnt[j] += colcnt[j - 1];
-    c.ktlp = colcnt;
+    const bool listed = famListed(c.Zk, n);
+    const int lanes = listed ? kFam : 1;
+    auto place = [&](int32_t k, int qq) { return static_cast<size_t>(c.ki[k]) * lanes + (listed ? c.kl[qq] : 0); };
+    std::vector<int32_t> at_col(static_cast<size_t>(n) * lanes + 1, 0);
+    for (int qq = 0; qq < c.K; ++qq)
+        for (int32_t k = c.kp[qq]; k < c.kp[qq + 1]; ++k) ++at_col[place(k, qq) + 1];
+    for (size_t j = 1; j < at_col.size(); ++j) at_col[j] += at_col[j - 1];
+    c.ktlp.clear();
+    if (listed) c.ktlp = at_col;
     c.ktp.resize(static_cast<size_t>(n) + 1);
-    for (int32_t j = 0; j <= n; ++j) c.ktp[j] = colcnt[static_cast<size_t>(j) * kFam];
+    for (int32_t j = 0; j <= n; ++j) c.ktp[j] = at_col[static_cast<size_t>(j) * lanes];
     c.ktr.resize(static_cast<size_t>(c.Zk));
     c.ktl.resize(static_cast<size_t>(c.Zk));
     c.ktv.resize(static_cast<size_t>(c.Zk));
-    for (int qq = 0; qq < c.K; ++qq)
+    for (int qq = 0; qq < c.K; ++qq)  // lane by lane
         for (int32_t k = c.kp[qq]; k < c.kp[qq + 1]; ++k) {
-            const int32_t at = colcnt[static_cast<size_t>(c.ki[k]) * kFam + c.kl[qq]]++;
+            const int32_t at = at_col[place(k, qq)]++;
             c.ktr[at] = qq;
             c.ktl[at] = c.kl[qq];
             c.ktv[at] = c.kv[k];
@@ -984,7 +995,7 @@ int32_t solveFamilyPack(FamPack& fp, const pdlpx_options& o, std::chrono::steady
     std::memcpy(I(fp.o_kfirst), cuts.kf.data(), 4 * cuts.kf.size());
     *reinterpret_cast<uint32_t*>(H + fp.o_live) = L >= kFam ? ~0u : ((1u << L) - 1u);
     std::memcpy(I(fp.o_ktptr), cuts.ktp.data(), 4 * cuts.ktp.size());
-    std::memcpy(I(fp.o_ktlptr), cuts.ktlp.data(), 4 * cuts.ktlp.size());
+    if (!cuts.ktlp.empty()) std::memcpy(I(fp.o_ktlptr), cuts.ktlp.data(), 4 * cuts.ktlp.size());
     std::memcpy(I(fp.o_ktrow), cuts.ktr.data(), 4 * cuts.ktr.size());
     std::memcpy(I(fp.o_ktlane), cuts.ktl.data(), 4 * cuts.ktl.size());
     std::memcpy(D(fp.o_ktval), cuts.ktv.data(), 8 * cuts.ktv.size());
@@ -1138,7 +1149,7 @@ int32_t solveFamilyPack(FamPack& fp, const pdlpx_options& o, std::chrono::steady
         a.K = fp.K;
         a.L = L;
         a.gk = fp.K > 0 ? famBlocks(fp.K) : 0;
-        a.listed = fp.Zk >= static_cast<int64_t>(kFamListed) * n;
+        a.listed = famListed(fp.Zk, n);
         a.nbk = L;  // one check block per lane for its appended rows (identity partials when it has none)
     };
     setShape(fp.args);
