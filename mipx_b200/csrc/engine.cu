@@ -2499,12 +2499,11 @@ int32_t Engine::solveDevice(pdlpx_result* out) {
     auto pickLinked = [&]() -> int {
         if (!d.linked) return 0;
         if (d.tiny != 0) return 1;
-        if (!link_share.fits()) return 0;
-        if (!d.link_try) return 1;
         const DeviceLp::Tried &a = d.tried[prec][0], &b = d.tried[prec][1];
-        if (!undecided()) return b.ms / b.iters < a.ms / a.iters ? 1 : 0;
-        if (cycle_ms > kAheadMs) return 0;
-        return b.iters < kTryIters ? 1 : 0;
+        const bool pays = !d.link_try || (!undecided() ? b.ms / b.iters < a.ms / a.iters
+                                                       : cycle_ms <= kAheadMs && b.iters < kTryIters);
+        link_share.set(pays ? d.link_warps : 0);  // the launches hold no share from other solvers' grids
+        return pays && link_share.fits() ? 1 : 0;
     };
     struct Queued {
         int prec, link;
