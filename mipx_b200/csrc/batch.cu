@@ -883,7 +883,7 @@ struct Pack {
     // linked cycle: cells and unit lists of the live LPs
     bool linkable = false;       // every side is sliced ELL and no option pins its launch shape
     bool linked = false;         // the live LPs are few enough
-    int link_lanes = 4, link_warps = 0;
+    int link_lanes = 4, link_warps = 0, link_share = 0;
     cudaGraphExec_t lcycle = nullptr;
     int lcycle_launches = 0;
     std::vector<int4> h_pu, h_du;
@@ -1213,7 +1213,7 @@ struct Pack {
     // uploaded on the pack's stream.
     cudaError_t planLinked(const std::vector<char>& keep, int device, int sms) {
         linked = false;
-        link_warps = 0;
+        link_warps = link_share = 0;
         if (!linkable) return cudaSuccess;
         int64_t z = 0, units4 = 0, units2 = 0;  // with 4 lanes per column and 8 per row; 2 and 4
         for (const Item* it : items)
@@ -1236,11 +1236,10 @@ struct Pack {
         }
         const int64_t total_units = static_cast<int64_t>(h_pu.size() + h_du.size());
         link_warps = static_cast<int>(std::min<int64_t>(warps_max, (total_units + sms - 1) / sms));
-        linked = cooperativeFits(linkedKernel(), device, sms, linkedGrid(sms), 32 * link_warps);
-        if (!linked) {
-            link_warps = 0;
-            return cudaSuccess;
-        }
+        int blocks = 0;
+        linked = cooperativeFits(linkedKernel(), device, sms, linkedGrid(sms), 32 * link_warps, blocks);
+        if (!linked) return cudaSuccess;
+        link_share = linkShareOf(blocks, linkTwice(total_units, sms));
         cudaError_t e = cudaMemcpyAsync(d + o_pu, h_pu.data(), sizeof(int4) * h_pu.size(), cudaMemcpyHostToDevice, s);
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(d + o_du, h_du.data(), sizeof(int4) * h_du.size(), cudaMemcpyHostToDevice, s);
@@ -1865,7 +1864,7 @@ int32_t solvePack(Pack& pk, const pdlpx_options& o, std::chrono::steady_clock::t
     // ---- restart cycles; finished LPs are read back after the cycle that ends them
     std::vector<char> keep(L, 1), collected(L, 0);
     if (!pk.persist) PDLPX_BCK(pk.planLinked(keep, dev, sms));
-    LinkShare share(dev, pk.link_warps);
+    LinkShare share(dev, pk.link_share);
     int perr = 0;
     SleepWait sleeper;
     std::vector<int> cl, rl;
@@ -1939,7 +1938,7 @@ int32_t solvePack(Pack& pk, const pdlpx_options& o, std::chrono::steady_clock::t
                 PDLPX_BCK(pk.uploadPersistTiles());
             else
                 PDLPX_BCK(pk.planLinked(keep, dev, sms));
-            share.set(pk.link_warps);
+            share.set(pk.link_share);
             for (cudaGraphExec_t* g : {&pk.cycle, &pk.lcycle}) {
                 if (*g) cudaGraphExecDestroy(*g);
                 *g = nullptr;

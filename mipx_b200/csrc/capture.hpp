@@ -48,8 +48,9 @@ inline bool residentAtOnce(int cooperative, int blocks_per_sm, int sms, int grid
     return cooperative != 0 && grid > 0 && static_cast<long long>(blocks_per_sm) * sms >= grid;
 }
 template <class... Args>
-bool cooperativeFits(void (*kernel)(Args...), int device, int sms, int grid, int threads) {
-    int coop = 0, blocks = 0;
+bool cooperativeFits(void (*kernel)(Args...), int device, int sms, int grid, int threads, int& blocks) {
+    int coop = 0;
+    blocks = 0;  // of the kernel that one SM holds
     const bool known = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) == cudaSuccess &&
                        cudaOccupancyMaxActiveBlocksPerMultiprocessor(
                            &blocks, reinterpret_cast<const void*>(kernel), threads, 0) == cudaSuccess;

@@ -614,6 +614,7 @@ struct DeviceLp {
     bool linked = false;
     int link_lanes = 4;
     int link_warps = 0;  // of its grid per SM
+    int link_share = 0;  // LinkShare
     bool link_refused = false;  // its launch failed on this image: the step launches run
     int tiny = 0;        // one block runs it (tiny.cuh): 1 short columns, 2 short rows
     int longestRow[2] = {0, 0};  // entries of the longest column / row that is not one of the long ones
@@ -1046,12 +1047,12 @@ int linkedGrid(const DeviceLp& d, int units) { return std::min(d.sms, (units + d
 // holds); columns of up to 3 entries take one lane (transportation 30 x 40: 2.6
 // against 2.8), long ones 8.  One block takes an LP whose slices are its warps and
 // whose entries fit their registers (tiny.cuh): 90 x 250 linked 2.3 -> 1.2.  No block
-// waits on another there, so it needs no share of the SMs (link_warps 0).
+// waits on another there, so it needs no share of the device.
 void planLinked(DeviceLp& d) {
     // rowDotU with two sums per lane (the autotuner may pick it) has no linked form
     auto supported = [](int shape) { return isSell(shape) || kShapes[shape].U >= kLinkU; };
     d.linked = d.link_x != nullptr && !d.link_refused && supported(d.shapeP) && supported(d.shapeD);
-    d.tiny = d.link_warps = 0;
+    d.tiny = d.link_warps = d.link_share = 0;
     d.link_try = false;
     if (!d.linked) return;
     if (!linkCsr(d) && (d.n + kSlice - 1) / kSlice + (d.m + kSlice - 1) / kSlice <= kTinyWarps) {
@@ -1080,13 +1081,16 @@ void planLinked(DeviceLp& d) {
         const int units = shape.P.units + shape.D.units;
         d.link_warps = std::min(linkThreads(linkCsr(d)) / 32, (units + d.sms - 1) / d.sms);
         shape.warps = d.sms * d.link_warps;
-        return cooperativeFits(kernel, d.device, d.sms, linkedGrid(d, units), 32 * d.link_warps);
+        int blocks = 0;
+        const bool fits = cooperativeFits(kernel, d.device, d.sms, linkedGrid(d, units), 32 * d.link_warps, blocks);
+        d.link_share = linkShareOf(blocks, !linkCsr(d) && linkTwice(units, d.sms));
+        return fits;
     };
     d.linked = withLinked<double>(d, plan) && (!d.mixed || withLinked<float>(d, plan));
     const LinkRule rule = linkRule(shape);
     if (rule == LinkRule::kNever) d.linked = false;
     d.link_try = rule == LinkRule::kTry;
-    if (!d.linked) d.link_warps = 0;
+    if (!d.linked) d.link_warps = d.link_share = 0;
 }
 
 template <class T>
@@ -2459,7 +2463,7 @@ int32_t Engine::solveDevice(pdlpx_result* out) {
         PDLPX_CK(cudaMemsetAsync(d.link_y, 0, sizeof(LinkCell<double>) * static_cast<size_t>(m), s));
     }
     // ---- capture the restart-cycle graphs lazily
-    LinkShare link_share(d.device, d.linked ? d.link_warps : 0);
+    LinkShare link_share(d.device, d.link_share);
     auto ensureCycle = [&](int prec, int link) -> cudaError_t {
         if (d.cycle[prec][link]) return cudaSuccess;
         return captureGraph(s, d.cycle[prec][link], [&] {
@@ -2502,7 +2506,7 @@ int32_t Engine::solveDevice(pdlpx_result* out) {
         const DeviceLp::Tried &a = d.tried[prec][0], &b = d.tried[prec][1];
         const bool pays = !d.link_try || (!undecided() ? b.ms / b.iters < a.ms / a.iters
                                                        : cycle_ms <= kAheadMs && b.iters < kTryIters);
-        link_share.set(pays ? d.link_warps : 0);  // the launches hold no share from other solvers' grids
+        link_share.set(pays ? d.link_share : 0);  // the launches hold no share from other solvers' grids
         return pays && link_share.fits() ? 1 : 0;
     };
     struct Queued {

@@ -25,6 +25,7 @@
 #pragma once
 
 #include <algorithm>
+#include <atomic>
 #include <cstdint>
 
 namespace pdlpx {
@@ -78,6 +79,46 @@ inline LinkRule linkRule(const LinkShape& s) {
     if (per_warp > 2 || rounds > 8 || std::min(x, y) > 500) return LinkRule::kNever;
     return x + y <= 2500 || serial >= 32 ? LinkRule::kTry : LinkRule::kNever;
 }
+
+// Share of a device that a solve's linked grid takes from the other solves on it.  As
+// many grids run side by side as one SM holds blocks of them; further ones wait, while
+// step launches of many solves overlap.  So a device takes grids up to that number,
+// twice as many where the linked cycle is twice as fast as the launches to begin
+// with; beyond, cycles run by launches (the same bits, so every cycle may choose).
+// Measured on B200 (us per iteration of all solves, 1, 2, 4, 8 solver threads):
+//   2,000 x 5,000 (two blocks per SM)  linked 3.4 2.1 2.0 2.1   launches 8.6 4.6 2.4 1.3
+//   6,000 x 15,000 (one)               linked 4.0 4.0 3.9 3.9   launches 9.3 5.0 2.7 1.7
+//   20,000 x 50,000 (one)              linked 8.5 8.3 8.3 8.3   launches 11.5 7.2 5.2 3.8
+//   transportation 97 x 131 (one)      linked 3.3 3.1 3.1 3.2   launches 5.5 3.0 1.6 0.9
+//   power law 2,000 x 8,000 (one)      linked 8.9 9.4 9.0 8.9   launches 15.7 8.2 4.3 2.3
+//   400 x 1,000 (eight)                linked 2.6 1.4 0.8 0.5   launches 7.3 3.9 2.1 1.1
+constexpr int kLinkFull = 1024;
+inline int linkShareOf(int blocks_per_sm, bool twice) {
+    return std::max(1, kLinkFull / (std::max(1, blocks_per_sm) * (twice ? 2 : 1)));
+}
+// At 1.5 units per warp of a full grid or fewer, both sides sliced ELL.
+inline bool linkTwice(std::int64_t units, int sms) { return 2 * units <= 3 * static_cast<std::int64_t>(sms) * 16; }
+
+inline std::atomic<int> g_link_share[64];  // by device
+class LinkShare {
+public:
+    LinkShare(int device, int share) : device_(device) { set(share); }
+    ~LinkShare() { set(0); }
+    LinkShare(const LinkShare&) = delete;
+    LinkShare& operator=(const LinkShare&) = delete;
+    // this solve's grid now takes `share`
+    void set(int share) {
+        if (device_ < 0 || device_ >= 64) return;
+        g_link_share[device_].fetch_add(share - share_, std::memory_order_relaxed);
+        share_ = share;
+    }
+    bool fits() const {
+        return share_ > 0 && g_link_share[device_].load(std::memory_order_relaxed) <= std::max(kLinkFull, share_);
+    }
+
+private:
+    int device_, share_ = 0;
+};
 
 // A pack of sliced-ELL LPs: lanes per column (twice as many per row) of its linked
 // cycle, 0 where the step launches run.  units4, units2: units of the live LPs with 4

@@ -35,9 +35,6 @@
 // groupSum) and updated by the same expressions: iterates are the same bits.
 #pragma once
 
-#include <algorithm>
-#include <atomic>
-
 #include "kernels.cuh"
 
 namespace pdlpx {
@@ -67,34 +64,6 @@ struct LinkTime {
     long long primal_clk, dual_clk;
     int iters;
     int pad;
-};
-
-// Warps per SM of the linked grids that the solves running on a device would
-// launch, by device.  Above kLinkShare of them a cycle runs by launches, which
-// share the SMs better than waiting grids do (16 solver threads on one B200, us
-// per LP-iteration of all: 2,000 x 5,000 launches 0.80, linked 2.05; with 4
-// threads 2.44 and 2.15).  Both give the same bits, so the choice is made anew
-// for every cycle.
-constexpr int kLinkShare = 32;
-inline std::atomic<int> g_link_warps[64];
-class LinkShare {
-public:
-    LinkShare(int device, int warps) : device_(device) { set(warps); }
-    ~LinkShare() { set(0); }
-    LinkShare(const LinkShare&) = delete;
-    LinkShare& operator=(const LinkShare&) = delete;
-    // this solve's grid now takes `warps` per SM
-    void set(int warps) {
-        if (device_ < 0 || device_ >= 64) return;
-        g_link_warps[device_].fetch_add(warps - warps_, std::memory_order_relaxed);
-        warps_ = warps;
-    }
-    bool fits() const {
-        return warps_ > 0 && g_link_warps[device_].load(std::memory_order_relaxed) <= std::max(kLinkShare, warps_);
-    }
-
-private:
-    int device_, warps_ = 0;
 };
 
 // ---- cells ---------------------------------------------------------------------

@@ -2,6 +2,8 @@
 // "never" where the launches are faster by 20 % or more, "always" where the linked
 // cycle is, "try" between.  Sizes and units are those of a device with 148 SMs.
 #include <cstdio>
+#include <memory>
+#include <vector>
 
 #include "link_plan.hpp"
 
@@ -38,7 +40,37 @@ static void pack(int want, const char* name, long long count, int m, int n, long
     ++bad;
 }
 
+// How many solves of one kind, one after another, find room.
+static int fitting(int share) {
+    std::vector<std::unique_ptr<LinkShare>> all;
+    for (int k = 0; k < 40; ++k) {
+        all.push_back(std::make_unique<LinkShare>(3, share));
+        if (!all.back()->fits()) return k;
+    }
+    return 40;
+}
+static void shares(int want, int got) {
+    if (want == got) return;
+    std::printf("FAIL %d solves instead of %d\n", got, want);
+    ++bad;
+}
+
 int main() {
+    shares(1, fitting(linkShareOf(1, false)));  // grids that fill the SMs, as CSR ones do
+    shares(2, fitting(linkShareOf(1, true)));
+    shares(4, fitting(linkShareOf(2, true)));
+    shares(8, fitting(linkShareOf(8, false)));
+    shares(0, fitting(0));  // no grid
+    {
+        LinkShare a(3, linkShareOf(1, false)), b(3, linkShareOf(1, false));
+        if (a.fits() || b.fits()) std::printf("FAIL two full grids\n"), ++bad;
+        b.set(0);  // runs by launches from now on
+        if (!a.fits()) std::printf("FAIL alone again\n"), ++bad;
+        LinkShare c(4, linkShareOf(1, false)), d(-1, 5), e(64, 5);
+        if (!c.fits() || d.fits() || e.fits()) std::printf("FAIL other devices\n"), ++bad;
+    }
+    shares(1, fitting(kLinkFull + 1));
+    if (!linkTwice(3552, 148) || linkTwice(3553, 148)) std::printf("FAIL units\n"), ++bad;
     pack(0, "no LP", 0, 50, 125, 930);
     pack(4, "12 of 1,000 x 2,500", 12, 1000, 2500, 20000);
     pack(2, "300 of 50 x 125", 300, 50, 125, 930);
