@@ -409,9 +409,11 @@ __global__ void __launch_bounds__(linkThreads(CSR), 1) linkedSteps(LinkArgs<T> a
 
 // The long columns as CSR rows of G lanes (blocks [0, lblocks)) and the short ones
 // in sliced ELL, in one launch: one after the other, each leaves SMs idle (a
-// mid-size LP's launches hold a few blocks per SM) and pays its own ramp.  The
-// gathers' sectors from L2 bound it then, 32 bytes each at 6-7 TB/s.  Same
-// per-thread work as the two launches.  Measured on B200 (power-law LPs, us per
+// mid-size LP's launches hold a few blocks per SM) and pays its own ramp.  What
+// bounds it then: latency at 25k x 100k (47 % of the warp slots, waiting on loads 11
+// of 17 cycles per instruction; L1 46 %, L2 8 % of their rates), L1's tag stage at
+// 200k x 700k and beyond (L1 71 %, L2 46 %, DRAM 23 %).  Same per-thread work as the
+// two launches.  Measured on B200 (power-law LPs, us per
 // iteration, apart -> in one): 25k x 100k 31.0 -> 21.9, 60k x 200k 38.1 -> 25.2,
 // 100k x 400k 54.2 -> 49.1, 200k x 700k 98.1 -> 73.9; 25k x 100k in FP64
 // 29.5 -> 21.7.
@@ -450,7 +452,8 @@ __global__ void __launch_bounds__(kBlock) powerASell(PowerArgs a, const int2* __
 // The short columns [begin, end) in sliced ELL, and in the first `lblocks`
 // blocks the long columns [0, begin) as CSR rows of G lanes: two launches in
 // one, so that neither trails off alone.  Bound by L1's tag stage, one scattered
-// sector per clock and SM: at 8 resident blocks (32 registers) 99 us on the
+// sector per clock and SM (200k x 800k: L1 83 %, L2 43 %, DRAM 16 % of their rates):
+// at 8 resident blocks (32 registers) 99 us on the
 // 500k x 2M power-law LP against 84 + 51 us apart (20.1M gathers are 69 us).
 // With the sums in powerNormalize an iteration there went from 250 to 211 us.
 template <int G, int U, class V>

@@ -15,7 +15,8 @@
 // 1,000 across, twice per iteration), the sum of a row in entry order (12 cycles
 // per entry), and L1's tag stage, which takes one of a warp's 32 scattered cells
 // per clock -- so a slice's rows are spread over several warps with 2-8 lanes
-// per row.  Measured (B200, FP64, us per iteration, the steps alone, launches ->
+// per row.  Counters at 2,000 x 5,000: L1 busy 50 % of the cycle, L2 32 %, DRAM
+// 0.03 %, loads waited for in 4 of 10 issue slots.  Measured (B200, FP64, us per iteration, the steps alone, launches ->
 // linked): 400 x 1,000 7.2 -> 2.5, 2,000 x 5,000 8.0 -> 3.0, 6,000 x 15,000
 // 8.7 -> 3.9, 20,000 x 50,000 10.3 -> 8.4.  (Before that: one 8-16 CTA cluster
 // with the vectors copied to every SM through distributed shared memory, 6.0 at
@@ -24,7 +25,8 @@
 // Why no cell is overwritten too early: x_j is read by the rows i with an entry
 // in column j, and column j's next value needs y_i of the same rows i, each of
 // which its owner publishes after its own reads (its value depends on them).
-// Padding entries (value 0) are not waited for and count as 0.
+// Entries of value 0 (padding among them) are not waited for and add nothing.  The
+// step kernels add 0 x[c] for theirs: the same bits while x is finite.
 // Why it always ends: a warp runs its columns' step k, then its rows' step k,
 // and waits only for cells of strictly earlier half-steps; every block is
 // resident (cooperative launch).  Should a block be kept from running all the
@@ -32,7 +34,7 @@
 // a launch that finds it set does nothing.
 //
 // Every row is summed in the order of the per-step kernels (sellDot, rowDotU +
-// groupSum) and updated by the same expressions: iterates are the same bits.
+// groupSum) and updated by the same expressions.  Which LPs it runs: link_plan.hpp.
 #pragma once
 
 #include "kernels.cuh"
