@@ -1025,7 +1025,7 @@ LinkSide<T> linkSide(const DeviceLp& d, const IterArgs<T>& ia, bool primal) {
 bool linkCsr(const DeviceLp& d) { return !isSell(d.shapeP) || !isSell(d.shapeD) || d.nlP > 0 || d.nlD > 0; }
 bool linkable(const DeviceLp& d, const pdlpx_options& o) {
     return d.lt_C == 0 && o.hot_cache <= 0 && o.shape_primal <= 0 && o.shape_dual <= 0 && o.spmv_group_a <= 0 &&
-           o.spmv_group_at <= 0 && d.nnz <= kLinkEntries;
+           o.spmv_group_at <= 0 && linkRoom(d.nnz, d.m, d.n);
 }
 // f(kernel, lanes per sliced-ELL column, lanes per sliced-ELL row) of the planned grid.
 template <class T, class F>
@@ -1620,7 +1620,7 @@ static int32_t buildDevice(std::unique_ptr<DeviceLp>& dp, const ScaledLp& sc_in,
     d.zlD = zlD;
     d.zlP = zlP;
     d.longest = std::max(d.nlD > 0 ? sc.a.ptr[1] : 0, d.nlP > 0 ? sc.at.ptr[1] : 0);  // the longest come first
-    if (nnz <= kLinkEntries) {
+    if (linkRoom(nnz, d.m, d.n)) {
         for (int32_t j = d.nlP; j < d.n; ++j) d.longestRow[0] = std::max(d.longestRow[0], sc.at.ptr[j + 1] - sc.at.ptr[j]);
         for (int32_t i = d.nlD; i < d.m; ++i) d.longestRow[1] = std::max(d.longestRow[1], sc.a.ptr[i + 1] - sc.a.ptr[i]);
     }

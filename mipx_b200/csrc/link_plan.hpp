@@ -45,6 +45,12 @@ struct LinkShape {
 };
 
 constexpr std::int64_t kLinkEntries = 600000;  // no LP beyond
+// Rows and columns likewise: their cells would take 16 bytes each for nothing, since
+// no LP of more than kLinkUnits units per warp gained (6.4 units 6.8 -> 6.9, 4.3 units
+// 14.7 -> 14.1).
+constexpr std::int64_t kLinkRows = 1000000;
+constexpr int kLinkUnits = 12;
+inline bool linkRoom(std::int64_t nnz, std::int64_t m, std::int64_t n) { return nnz <= kLinkEntries && m + n <= kLinkRows; }
 
 enum class LinkRule { kNever, kTry, kAlways };
 
@@ -55,7 +61,7 @@ inline int linkRounds(int longest, int lanes) {
 
 inline LinkRule linkRule(const LinkShape& s) {
     const bool csr = s.P.lanes > 0 || s.D.lanes > 0, longs = s.P.nl > 0 || s.D.nl > 0;
-    if (s.longest > 1000) return LinkRule::kNever;
+    if (s.longest > 1000 || s.P.units + s.D.units > static_cast<std::int64_t>(kLinkUnits) * s.warps) return LinkRule::kNever;
     if (!csr && !longs) {
         if (s.nnz <= 150000 && s.P.rows + s.D.rows <= 60000) return LinkRule::kAlways;
         return s.nnz <= kLinkEntries ? LinkRule::kTry : LinkRule::kNever;

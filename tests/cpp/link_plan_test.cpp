@@ -90,6 +90,10 @@ int main() {
     expect(maybe, "5,798 x 29,377", 322000, 5798, 29377, 0, 0, 15, 84, 2, 4);
     expect(maybe, "30,000 x 75,000", 600000, 30000, 75000, 0, 0, 12, 37, 2, 4);
     expect(never, "one entry more", 600001, 30000, 75000, 0, 0, 12, 37, 2, 4);
+    expect(maybe, "100,000 x 100,000", 551506, 100000, 100000, 0, 0, 10, 18, 2, 4);
+    expect(never, "200,000 x 100,000", 400000, 200000, 100000, 0, 0, 8, 8, 4, 8);
+    if (!linkRoom(600000, 500000, 500000) || linkRoom(600000, 500001, 500000) || linkRoom(600001, 1, 1))
+        std::printf("FAIL room\n"), ++bad;
     // long columns or rows beside it
     expect(always, "power law 3,039 x 4,575", 45000, 3039, 4575, 0, 0, 64, 30, 4, 8, 101, 0, 289);
     expect(maybe, "power law 4,203 x 6,843", 65000, 4203, 6843, 0, 0, 64, 32, 4, 8, 134, 0, 360);
